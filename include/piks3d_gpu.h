@@ -228,17 +228,18 @@ enum { PIKS_PREC_FP64 = 0, PIKS_PREC_FP32 = 1 };
 piks_status piks_set_precision(piks_ctx *ctx, int32_t precision);
 piks_status piks_get_precision(piks_ctx *ctx, int32_t *precision);
 
-/* Sweep schedule. The default cuts the box into 8x4x4 tiles (4x4x4 when the context is in
- * FP32 at setup) and sweeps, for each octant,
- * the tiles in diagonal order, each tile's local hyperplanes in shared memory (one launch
- * per tile diagonal). tx = 0 selects the per-node hyperplane schedule (one launch per
- * voxel hyperplane u+v+w). Both give identical results; the tile schedule also falls back
- * to the per-node one when a tile needs more rows than shared memory holds. Takes effect
+/* Sweep schedule. The default marches columns of each octant along its hyperplanes
+ * (PIKS_SCHED_WAVE below). A tile shape set here selects the tile schedule instead: the box
+ * is cut into tx x ty x tz tiles (defaults 8x4x4, 4x4x4 when the context is in FP32 at setup)
+ * and each octant's tiles are swept in diagonal order, each tile's local hyperplanes in shared
+ * memory (one launch per tile diagonal). tx = 0 selects the per-node hyperplane schedule (one
+ * launch per voxel hyperplane u+v+w). All give identical results; a schedule that needs more
+ * rows than shared memory holds falls back to the next (columns, tiles, nodes). Takes effect
  * at the next piks_setup_physical_grid. No counterpart in the reference (its sweep is a
  * serial raster loop per octant). */
 piks_status piks_set_tiles(piks_ctx *ctx, int32_t tx, int32_t ty, int32_t tz);
-/* How the tile jobs are launched: PIKS_SCHED_TILE_DIAGONALS (default) launches each tile
- * diagonal separately; PIKS_SCHED_TILE_DATAFLOW runs all jobs of an iteration in one
+/* How the tile jobs are launched: PIKS_SCHED_TILE_DIAGONALS launches each tile diagonal
+ * separately (the default once a tile shape was set); PIKS_SCHED_TILE_DATAFLOW runs all jobs of an iteration in one
  * launch, each job waiting for its upwind neighbour tiles through device flags (waits give
  * up after about a second: piks_synchronize / piks_chk_converge then return
  * PIKS_ERR_CUDA); PIKS_SCHED_TILE_COLUMNS runs one persistent launch in which each CTA
@@ -248,10 +249,14 @@ piks_status piks_set_tiles(piks_ctx *ctx, int32_t tx, int32_t ty, int32_t tz);
  * next (waits give up after about two seconds, reported as for the dataflow launch);
  * PIKS_SCHED_TILE_PIPELINED runs the same producer / consumer kernel over single jobs taken
  * in diagonal order, each job's upwind rows staged from HBM once their jobs are done, the
- * producer up to three jobs ahead. A change between launch schedules that read different
- * forms of the tile jobs rebuilds them. All give identical values. */
+ * producer up to three jobs ahead; PIKS_SCHED_WAVE (the default without a tile shape) does not
+ * use tiles: one persistent launch whose CTAs each march a column of an octant (a small
+ * cross-section in x and y over the whole z extent) along the hyperplanes u+v+w, rows in a
+ * shared-memory ring, waiting for the upwind columns' published hyperplanes (waits as for the
+ * column launch). A change between launch schedules that read different forms of the jobs
+ * rebuilds them. All give identical values. */
 enum { PIKS_SCHED_TILE_DATAFLOW = 0, PIKS_SCHED_TILE_DIAGONALS = 1, PIKS_SCHED_TILE_COLUMNS = 2,
-       PIKS_SCHED_TILE_PIPELINED = 3 };
+       PIKS_SCHED_TILE_PIPELINED = 3, PIKS_SCHED_WAVE = 4 };
 piks_status piks_set_schedule(piks_ctx *ctx, int32_t schedule);
 /* Autotuner of the sweep schedule: right after piks_setup_physical_grid (before the first
  * iteration) times `sweeps` sweeps of each candidate (4 int32 each: TX, TY, TZ, launch
@@ -260,7 +265,7 @@ piks_status piks_set_schedule(piks_ctx *ctx, int32_t schedule);
  * milliseconds per sweep of each candidate (-1 where a candidate does not apply). */
 piks_status piks_autotune(piks_ctx *ctx, const int32_t *candidates, int32_t ncand, int32_t sweeps,
                           int32_t *chosen, double *ms_out);
-/* [tile schedule in use (0/1), TX, TY, TZ, largest shared-memory slot count of a job,
+/* [columns or tiles in use (0: the per-node schedule), TX, TY, TZ, largest shared-memory slot count of a job,
  *  launch schedule, number of jobs] */
 piks_status piks_get_schedule(piks_ctx *ctx, int32_t *out, int32_t n);
 

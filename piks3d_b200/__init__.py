@@ -150,7 +150,7 @@ def _dptr(a):
 
 
 PREC_FP64, PREC_FP32 = 0, 1
-SCHED_TILE_DATAFLOW, SCHED_TILE_DIAGONALS, SCHED_TILE_COLUMNS, SCHED_TILE_PIPELINED = 0, 1, 2, 3
+SCHED_TILE_DATAFLOW, SCHED_TILE_DIAGONALS, SCHED_TILE_COLUMNS, SCHED_TILE_PIPELINED, SCHED_WAVE = 0, 1, 2, 3, 4
 PREP_HOST, PREP_DEVICE = 0, 1
 
 KERNEL_NAMES = ("sweep", "commit", "capture", "walls", "inlet_outlet", "symmetry", "moments", "flux")

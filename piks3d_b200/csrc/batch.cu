@@ -22,17 +22,27 @@ struct piks_batch {
   std::vector<piks_ctx *> members;
   std::vector<int> versions;     // members' state versions at the last rebuild
   bool dirty = true;
+  // members swept by one launch: of one precision and chunk width, on tile jobs (items int2)
+  // or hyperplane columns (`wave`, items int4)
   struct Class {
-    bool fp32 = false;
+    bool fp32 = false, wave = false;
     int V = 0, slots = 0, tasks = 0, stride = 0;
+    WaveRings rings{0, 0, 0};
     std::vector<int2> items;
-    int2 *d_items = nullptr;
-    size_t cap = 0;
+    std::vector<int4> witems;
+    void *d_items = nullptr;
+    size_t cap = 0;              // bytes
+    const void *data() const { return wave ? (const void *)witems.data() : (const void *)items.data(); }
+    size_t bytes() const { return wave ? witems.size() * sizeof(int4) : items.size() * sizeof(int2); }
   };
   std::vector<Class> classes;
   DevState *d_states = nullptr;
   size_t states_cap = 0;
   int *d_ctl = nullptr;          // [class counters ..., error flag], kMaxClasses + 1
+  // the column classes' item counters (kMaxClasses), then the members' progress arrays;
+  // cleared before each sweep
+  int *d_prog = nullptr;
+  size_t prog_cap = 0, prog_n = 0;  // allocated, in use (ints)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int warm = 0;                  // iterations run since the last rebuild
   double *h_mass = nullptr;      // pinned, one per member
@@ -45,7 +55,7 @@ struct piks_batch {
 
 namespace {
 
-constexpr int kMaxClasses = 8;
+constexpr int kMaxClasses = 64;
 // Side streams for the members' boundary chains (more gives the graph no further overlap:
 // a boundary chain is a handful of dependent launches of a few microseconds each).
 constexpr int kMaxSide = 16;
@@ -92,6 +102,24 @@ piks_status rebuild(piks_batch *b) {
   }
   std::vector<DevState> hs(nm);
   for (size_t m = 0; m < nm; ++m) hs[m] = b->members[m]->ds;
+  size_t prog = kMaxClasses;
+  for (size_t m = 0; m < nm; ++m)
+    if (b->members[m]->use_wave) prog += (size_t)hs[m].wv.ncol * hs[m].wv.nchunk;
+  if (prog > b->prog_cap) {
+    if (b->d_prog) cudaFree(b->d_prog);
+    b->d_prog = nullptr;
+    b->prog_cap = 0;
+    piks_status st = cuda_check(cudaMalloc(&b->d_prog, prog * sizeof(int)), "batch progress");
+    if (st) return st;
+    b->prog_cap = prog;
+  }
+  b->prog_n = prog;
+  prog = kMaxClasses;
+  for (size_t m = 0; m < nm; ++m)
+    if (b->members[m]->use_wave) {
+      hs[m].wv.progress = b->d_prog + prog;
+      prog += (size_t)hs[m].wv.ncol * hs[m].wv.nchunk;
+    }
   if (nm) {
     piks_status st = cuda_check(cudaMemcpyAsync(b->d_states, hs.data(), nm * sizeof(DevState), cudaMemcpyHostToDevice,
                                                 b->stream), "batch states upload");
@@ -102,27 +130,51 @@ piks_status rebuild(piks_batch *b) {
   for (size_t m = 0; m < nm; ++m) {
     const piks_ctx *c = b->members[m];
     const bool f32 = c->prec == PIKS_PREC_FP32;
-    const int V = tile_sweep_velocities(c->vel.Nc8, f32);
+    const int V = c->use_wave ? wave_velocities(c->vel.Nc8, f32) : tile_sweep_velocities(c->vel.Nc8, f32);
+    // (column members whose rings, records and lists together exceed a CTA's shared memory
+    // go to launches of their own)
+    auto joint = [&](const WaveRings &q) {
+      return WaveRings{std::max(q.ring, c->wave.ring), std::max(q.task_ring, c->wave.task_ring), std::max(q.max_rows, c->wave.max_rows)};
+    };
+    auto fits = [&](const piks_batch::Class &q) {
+      if (q.fp32 != f32 || q.wave != c->use_wave || q.V != V) return false;
+      const WaveRings j = joint(q.rings);
+      return !q.wave || wave_max_ring(c->vel.Nc8, f32, j.task_ring, j.max_rows) >= j.ring;
+    };
     int k = 0;
-    while (k < (int)cls.size() && !(cls[k].fp32 == f32 && cls[k].V == V)) ++k;
+    while (k < (int)cls.size() && !fits(cls[k])) ++k;
     if (k == (int)cls.size()) {
       if (k == kMaxClasses) return fail(PIKS_ERR_ARG, "batch: too many precision / velocity classes");
       piks_batch::Class nc;
       nc.fp32 = f32;
       nc.V = V;
+      nc.wave = c->use_wave;
       cls.push_back(nc);
     }
     cls_of[m] = k;
+    if (c->use_wave) {
+      cls[k].rings = joint(cls[k].rings);
+      continue;
+    }
     cls[k].slots = std::max(cls[k].slots, c->tiles.max_rows);
     cls[k].tasks = std::max(cls[k].tasks, c->tiles.max_tasks);
     cls[k].stride = std::max(cls[k].stride, c->tiles.steps_stride);
   }
   int maxdiag = 0;
-  for (auto *c : b->members) maxdiag = std::max(maxdiag, (int)c->tiles.launch_diag_end.size());
+  for (auto *c : b->members)
+    maxdiag = std::max(maxdiag, c->use_wave ? c->wave.diag.empty() ? 0 : c->wave.diag.back() + 1
+                                            : (int)c->tiles.launch_diag_end.size());
+  std::vector<size_t> at(nm, 0);                 // columns listed so far
   for (int d = 0; d < maxdiag; ++d)
     for (size_t m = 0; m < nm; ++m) {
       const piks_ctx *c = b->members[m];
       const TileJobs &tj = c->tiles;
+      if (c->use_wave) {
+        auto &witems = cls[(size_t)cls_of[m]].witems;
+        for (; at[m] < c->wave.diag.size() && c->wave.diag[at[m]] == d; ++at[m])
+          for (int ch = 0; ch < hs[m].wv.nchunk; ++ch) witems.push_back(make_int4((int)m, c->wave.col_list[at[m]], ch, 0));
+        continue;
+      }
       if (d >= (int)tj.launch_diag_end.size()) continue;
       const int l0 = d ? tj.launch_diag_end[(size_t)d - 1] : 0, l1 = tj.launch_diag_end[(size_t)d];
       const int nchunk = c->vel.Nc8 / cls[(size_t)cls_of[m]].V;
@@ -133,19 +185,19 @@ piks_status rebuild(piks_batch *b) {
     }
   // keep the device buffers of the old classes where they fit
   for (size_t k = 0; k < cls.size(); ++k) {
-    if (k < b->classes.size() && b->classes[k].cap >= cls[k].items.size()) {
+    const size_t need = std::max<size_t>(16, cls[k].bytes());
+    if (k < b->classes.size() && b->classes[k].cap >= need) {
       cls[k].d_items = b->classes[k].d_items;
       cls[k].cap = b->classes[k].cap;
       b->classes[k].d_items = nullptr;
     } else {
-      piks_status st = cuda_check(cudaMalloc(&cls[k].d_items, std::max<size_t>(1, cls[k].items.size()) * sizeof(int2)),
-                                  "batch items");
+      piks_status st = cuda_check(cudaMalloc(&cls[k].d_items, need), "batch items");
       if (st) return st;
-      cls[k].cap = std::max<size_t>(1, cls[k].items.size());
+      cls[k].cap = need;
     }
-    if (!cls[k].items.empty()) {
-      piks_status st = cuda_check(cudaMemcpyAsync(cls[k].d_items, cls[k].items.data(), cls[k].items.size() * sizeof(int2),
-                                                  cudaMemcpyHostToDevice, b->stream), "batch items upload");
+    if (cls[k].bytes()) {
+      piks_status st = cuda_check(cudaMemcpyAsync(cls[k].d_items, cls[k].data(), cls[k].bytes(), cudaMemcpyHostToDevice,
+                                                  b->stream), "batch items upload");
       if (st) return st;
     }
   }
@@ -163,13 +215,22 @@ piks_status rebuild(piks_batch *b) {
 // One iteration of every member, on the batch stream; `parity` offsets the members'
 // iteration numbers (0 = their next iteration, 1 = the one after).
 void enqueue_batch_iteration(piks_batch *b, int parity) {
+  bool wave = false;
   for (piks_ctx *c : b->members) {
+    wave |= c->use_wave;
+    if (c->use_wave) continue;
     const int nchunk_max = c->vel.Nc8 / 8 > 0 ? c->vel.Nc8 / 8 : 1;
     cudaMemsetAsync(c->ds.tv.flags, 0, (size_t)c->ds.tv.njobs * nchunk_max * sizeof(int), b->stream);
   }
+  if (wave) cudaMemsetAsync(b->d_prog, 0, b->prog_n * sizeof(int), b->stream);
   for (size_t k = 0; k < b->classes.size(); ++k) {
     const auto &cl = b->classes[k];
-    launch_tile_sweep_batch(b->d_states, cl.d_items, (int)cl.items.size(), cl.fp32, cl.V, cl.slots, cl.tasks,
+    if (cl.wave) {
+      launch_wave_sweep_batch(b->d_states, static_cast<const int4 *>(cl.d_items), (int)cl.witems.size(), cl.fp32, cl.V,
+                              cl.rings, b->d_prog + k, b->d_ctl + kMaxClasses, b->stream);
+      continue;
+    }
+    launch_tile_sweep_batch(b->d_states, static_cast<const int2 *>(cl.d_items), (int)cl.items.size(), cl.fp32, cl.V, cl.slots, cl.tasks,
                             cl.stride, b->d_ctl + k, b->d_ctl + kMaxClasses, b->stream);
   }
   const size_t ns = std::min(b->side.size(), b->members.size());
@@ -216,7 +277,7 @@ piks_status piks_batch_add(piks_batch *b, piks_ctx *c) {
   if (!b || !c) return fail(PIKS_ERR_ARG, "null argument");
   if (!c->have_geometry) return fail(PIKS_ERR_STATE, "batch member has no device state");
   if (c->device != b->device) return fail(PIKS_ERR_ARG, "batch member lives on another device");
-  if (!c->use_tiles) return fail(PIKS_ERR_ARG, "batch members need the tile schedule");
+  if (!c->use_tiles && !c->use_wave) return fail(PIKS_ERR_ARG, "batch members need the column or the tile schedule");
   if (c->setup.nranks > 1) return fail(PIKS_ERR_ARG, "a slab of a decomposed box cannot join a batch");
   if (b->members.size() >= 4096) return fail(PIKS_ERR_ARG, "batch holds at most 4096 members");
   if (std::find(b->members.begin(), b->members.end(), c) != b->members.end()) return PIKS_OK;
@@ -326,6 +387,7 @@ piks_status piks_batch_destroy(piks_batch *b) {
     if (cl.d_items) cudaFree(cl.d_items);
   if (b->d_states) cudaFree(b->d_states);
   if (b->d_ctl) cudaFree(b->d_ctl);
+  if (b->d_prog) cudaFree(b->d_prog);
   if (b->h_mass) cudaFreeHost(b->h_mass);
   for (size_t k = 0; k < b->side.size(); ++k) {
     cudaStreamDestroy(b->side[k]);

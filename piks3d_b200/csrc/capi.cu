@@ -113,15 +113,15 @@ piks_status alloc_state(piks_ctx *c, int prec) {
   const StateSizes z = state_sizes(c);
   piks_status st;
   if (prec == PIKS_PREC_FP64) {
-    if ((st = zeros(c, z.h, &s.h))) return st;
-    if ((st = zeros(c, z.fw, &s.fw))) return st;
+    if ((st = zeros(c, z.h + z.fw, &s.h))) return st;
+    s.fw = s.h + z.h;  // one row space: the columns' row lists index both
     for (int b = 0; b < 2; ++b) {
       if ((st = zeros(c, z.plane, &s.ghostW[b]))) return st;
       if ((st = zeros(c, z.plane, &s.ghostE[b]))) return st;
     }
   } else {
-    if ((st = zeros(c, z.h, &s.h32))) return st;
-    if ((st = zeros(c, z.fw, &s.fw32))) return st;
+    if ((st = zeros(c, z.h + z.fw, &s.h32))) return st;
+    s.fw32 = s.h32 + z.h;  // one row space: the columns' row lists index both
     for (int b = 0; b < 2; ++b) {
       if ((st = zeros(c, z.plane, &s.ghostW32[b]))) return st;
       if ((st = zeros(c, z.plane, &s.ghostE32[b]))) return st;
@@ -142,7 +142,7 @@ piks_status alloc_state(piks_ctx *c, int prec) {
 void free_state(piks_ctx *c, int prec) {
   DevState &s = c->ds;
   if (prec == PIKS_PREC_FP64) {
-    release(c, s.h); release(c, s.fw);
+    release(c, s.h);
     for (int b = 0; b < 2; ++b) { release(c, s.ghostW[b]); release(c, s.ghostE[b]); s.ghostW[b] = s.ghostE[b] = nullptr; }
     s.h = s.fw = nullptr;
     for (int side = 0; side < 2; ++side) {
@@ -151,7 +151,7 @@ void free_state(piks_ctx *c, int prec) {
       s.hrecv[side] = nullptr;
     }
   } else {
-    release(c, s.h32); release(c, s.fw32);
+    release(c, s.h32);
     for (int b = 0; b < 2; ++b) { release(c, s.ghostW32[b]); release(c, s.ghostE32[b]); s.ghostW32[b] = s.ghostE32[b] = nullptr; }
     s.h32 = s.fw32 = nullptr;
     for (int side = 0; side < 2; ++side) {
@@ -199,12 +199,13 @@ void drain_timing(piks_ctx *c) {
 // The tile sweeps' error flag: set when a dependency wait or a staging wait gave up (the
 // values of that sweep are then not the solver's).
 piks_status check_sweep_error(piks_ctx *c) {
-  if (!c->use_tiles || !c->ds.tv.err) return PIKS_OK;
+  const int *flag = c->use_wave ? c->ds.wv.err : c->use_tiles ? c->ds.tv.err : nullptr;
+  if (!flag) return PIKS_OK;
   int e = 0;
-  piks_status st = cuda_check(cudaMemcpyAsync(&e, c->ds.tv.err, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "err D2H");
+  piks_status st = cuda_check(cudaMemcpyAsync(&e, flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "err D2H");
   if (!st) st = cuda_check(cudaStreamSynchronize(c->stream), "err sync");
   if (st) return st;
-  if (e) return fail(PIKS_ERR_CUDA, "tile sweep: a dependency wait timed out");
+  if (e) return fail(PIKS_ERR_CUDA, "sweep: a dependency wait timed out");
   return PIKS_OK;
 }
 
@@ -239,7 +240,9 @@ void enqueue_sweep(piks_ctx *c, cudaStream_t st, int n) {
   const bool f32 = c->prec == PIKS_PREC_FP32;
   {
     Timed t(c, KT_SWEEP);
-    if (c->use_tiles && c->tiles.split) {
+    if (c->use_wave) {
+      launch_wave_sweep(s, f32, st);
+    } else if (c->use_tiles && c->tiles.split) {
       if (c->tiles.columns) launch_tile_sweep_columns(s, f32, 1, st);
       else launch_tile_sweep_pipelined(s, f32, 1, st);
     } else if (c->use_tiles && c->schedule == PIKS_SCHED_TILE_DATAFLOW) {
@@ -336,9 +339,98 @@ bool build_tiles_for(const piks_ctx *c, const int *dims, int form, TileJobs &tj,
   return ok;
 }
 
+// The hyperplane-column schedule of the context's geometry (false: not usable). The columns'
+// cross-section: a batch (one hyperplane of a column) costs some 1100 cycles whatever its size,
+// which asks for wide columns, and its rows fill the ring of one SM's shared memory, which has to
+// hold three of the largest batches and wants some to spare for the loads of the next. With rows
+// of 256 bytes (FP64 32, FP32 64 velocities) that is about 700 rows: 10 x 10, or 9 x 9 where most
+// of the box is pore space and most batches are full. Sweep per iteration on B200: 128^3 pack of
+// porosity 0.40, FP64, 8 x 8 / 10 x 10 / 12 x 12 3.42 / 2.87 / 2.93 ms, FP32 1.71 / 1.48 / 1.67;
+// 100^3 quarter sphere of porosity 0.75, FP64, 8 x 8 / 9 x 9 / 10 x 10 2.50 / 2.54 / 2.69 ms (the
+// tile diagonals 5.31, 2.66 and 5.58 ms). Octants of 8 velocities have rows of a quarter of that
+// and take 12 x 12 (96^3 pack, FP32, 8 x 8 / 10 x 10 / 12 x 12 / 16 x 16: 0.52 / 0.41 / 0.33 / 0.33 ms).
+bool build_wave(piks_ctx *c) {
+  c->wave = WaveJobs{};
+  const int Nc8 = c->vel.Nc8;
+  // every context reserves the records and lists of full columns of the widest cross-section,
+  // so that the members of a batch, whose launch takes the largest of each, fit together
+  const int wide = Nc8 <= 8 ? 12 : 10;
+  auto ring = [Nc8, wide](int task_ring, int max_rows) {
+    task_ring = std::max(task_ring, 3 * kWaveGroup * wide * wide);
+    max_rows = std::max(max_rows, 2 * kWaveGroup * wide * wide);
+    return std::min(wave_max_ring(Nc8, false, task_ring, max_rows), wave_max_ring(Nc8, true, task_ring, max_rows));
+  };
+  const Geometry &g = c->geo;
+  const double box = (double)(g.xu - g.xl + 1) * g.Ny * g.Nz;
+  for (int edge = Nc8 <= 8 || g.NF < 0.6 * box ? wide : wide - 1; edge >= 4; edge -= 2)
+    if (build_wave_jobs(g, edge, edge, ring, c->wave)) return true;
+  c->wave = WaveJobs{};
+  return false;
+}
+
+// The tile jobs of a context that iterates the hyperplane columns, built for the calls that
+// report or use them.
+void ensure_tiles(piks_ctx *c) {
+  if (c->use_wave && c->tiles.row_count.empty() && c->tile_dims[0] > 0)
+    build_tiles_for(c, c->tile_dims, TILE_FORM_SLOTS, c->tiles, c->prec);
+}
+
 bool build_tiles(piks_ctx *c) {
+  c->use_wave = false;
   c->use_tiles = build_tiles_for(c, c->tile_dims, tile_form(c->schedule), c->tiles, c->prec);
   return c->use_tiles;
+}
+
+// The velocity chunks and items of the columns for the state's precision.
+void wave_precision(piks_ctx *c) {
+  WaveView &w = c->ds.wv;
+  const bool f32 = c->prec == PIKS_PREC_FP32;
+  const int V = wave_velocities(c->vel.Nc8, f32);
+  w.nchunk = (c->vel.Nc8 + V - 1) / V;
+  w.items = c->wave_items[f32 ? 1 : 0];
+}
+
+// Device copy of the hyperplane-column schedule (replacing an earlier one).
+piks_status upload_wave(piks_ctx *c) {
+  WaveView &w = c->ds.wv;
+  for (const void *p : {(const void *)w.rows, (const void *)w.tasks, (const void *)w.batch, (const void *)w.cols,
+                        (const void *)w.counter, (const void *)c->wave_items[0], (const void *)c->wave_items[1]})
+    if (p) release(c, const_cast<void *>(p));
+  w = WaveView{};
+  c->wave_items[0] = c->wave_items[1] = nullptr;
+  if (!c->use_wave) return PIKS_OK;
+  const WaveJobs &wj = c->wave;
+  piks_status st;
+  int32_t *pi = nullptr;
+  if ((st = upload(c, wj.rows, &pi))) return st;
+  w.rows = pi;
+  if ((st = upload(c, wj.tasks, &pi))) return st;
+  w.tasks = reinterpret_cast<const int4 *>(pi);
+  if ((st = upload(c, wj.batch, &pi))) return st;
+  w.batch = reinterpret_cast<const int4 *>(pi);
+  if ((st = upload(c, wj.cols, &pi))) return st;
+  w.cols = reinterpret_cast<const int4 *>(pi);
+  int most = 1;
+  std::vector<int4> items;
+  for (int f32 = 0; f32 < 2; ++f32) {
+    const int V = wave_velocities(c->vel.Nc8, f32 != 0), n = (c->vel.Nc8 + V - 1) / V;
+    items.clear();
+    for (int32_t col : wj.col_list)
+      for (int k = 0; k < n; ++k) items.push_back(make_int4(0, col, k, 0));
+    most = std::max(most, n);
+    if ((st = upload(c, items, &c->wave_items[f32]))) return st;
+    if ((st = cuda_check(cudaStreamSynchronize(c->stream), "wave items"))) return st;  // `items` is reused
+  }
+  int *pw = nullptr;
+  if ((st = zeros(c, (size_t)wj.ncol * most + 8, &pw))) return st;
+  w.counter = pw;                 // the progress array follows it, the error flag comes last
+  w.progress = pw + 4;
+  w.err = pw + 4 + (size_t)wj.ncol * most;
+  w.ncol = wj.ncol;
+  w.A = wj.A; w.B = wj.B;
+  w.ring = wj.ring; w.task_ring = wj.task_ring; w.max_rows = wj.max_rows;
+  wave_precision(c);
+  return PIKS_OK;
 }
 
 // Device copy of the tile schedule (replacing an earlier one), with zeroed dataflow flags.
@@ -353,7 +445,8 @@ piks_status upload_tiles(piks_ctx *c) {
     if (p) release(c, const_cast<void *>(p));
   tv = TileView{};
   piks_status st;
-  if (!c->use_tiles) {
+  if (c->use_wave && c->tiles.row_count.empty()) return PIKS_OK;
+  if (!c->use_tiles && !c->use_wave) {
     // the per-node hyperplane sweep reads the task list (uploaded once, only if needed)
     if (!c->ds.tasks) {
       int32_t *pt = nullptr;
@@ -540,7 +633,11 @@ piks_status piks_setup_physical_grid(piks_ctx *c, const uint8_t *raw, int64_t nb
   c->have_host_geometry = true;
   c->tiles_tuned = false;
   if (!c->tiles_explicit) default_tile_dims(c->prec, c->tile_dims);
-  build_tiles(c);
+  c->tiles = TileJobs{};
+  c->use_tiles = false;
+  c->wave_items[0] = c->wave_items[1] = nullptr;
+  c->use_wave = c->schedule == PIKS_SCHED_WAVE && build_wave(c);
+  if (!c->use_wave) build_tiles(c);
   if (c->device < 0) {
     c->setup_seconds[3] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_setup).count();
     return PIKS_OK;
@@ -633,7 +730,7 @@ piks_status piks_setup_physical_grid(piks_ctx *c, const uint8_t *raw, int64_t nb
     }
   }
 #undef UP
-  if ((st = upload_tiles(c))) return st;
+  if ((st = c->use_wave ? upload_wave(c) : upload_tiles(c))) return st;
   s.nWall = g.nWall;
   s.ncommit = (int)(g.commit.size() / 3);
   s.nsym = (int)g.sym_node.size();
@@ -1020,6 +1117,14 @@ piks_status piks_set_precision(piks_ctx *c, int32_t precision) {
   if (st) return st;
   free_state(c, c->prec);
   c->prec = precision;
+  if (c->use_wave) {
+    // the columns serve both precisions
+    wave_precision(c);
+    if (!c->tiles_explicit) {
+      default_tile_dims(precision, c->tile_dims);
+      c->tiles = TileJobs{};
+    }
+  }
   if (c->use_tiles && !c->tiles_explicit && !c->tiles_tuned && (st = retile_for_precision(c))) return st;
   if (c->use_tiles && !c->tiles.split && c->tiles.plan_prec != precision) {
     // the schedule stayed: its launch plan becomes the new precision's
@@ -1037,16 +1142,21 @@ piks_status piks_set_tiles(piks_ctx *c, int32_t tx, int32_t ty, int32_t tz) {
     return fail(PIKS_ERR_ARG, "tile extents must be 0 (per-node schedule) or >= 2 with at most 65535 voxels");
   c->tile_dims[0] = tx; c->tile_dims[1] = tx ? ty : 0; c->tile_dims[2] = tx ? tz : 0;
   c->tiles_explicit = true;
+  // a tile shape selects the tile schedule (a shape of 0 the per-node one), unless a launch
+  // schedule was asked for by name
+  if (!c->schedule_explicit) c->schedule = PIKS_SCHED_TILE_DIAGONALS;
   return PIKS_OK;
 }
 
 piks_status piks_set_schedule(piks_ctx *c, int32_t schedule) {
   if (!c) return fail(PIKS_ERR_ARG, "null context");
-  if (schedule < PIKS_SCHED_TILE_DATAFLOW || schedule > PIKS_SCHED_TILE_PIPELINED)
+  if (schedule < PIKS_SCHED_TILE_DATAFLOW || schedule > PIKS_SCHED_WAVE)
     return fail(PIKS_ERR_ARG, "unknown schedule");
   const int old_form = tile_form(c->schedule);
   c->schedule = schedule;
-  if (old_form == tile_form(schedule) || !c->have_host_geometry) return PIKS_OK;
+  c->schedule_explicit = true;
+  const bool wave = schedule == PIKS_SCHED_WAVE;
+  if ((old_form == tile_form(schedule) && wave == c->use_wave) || !c->have_host_geometry) return PIKS_OK;
   // the new launch schedule reads another form of the tile jobs: rebuild them
   drop_tiles_next(c);
   if (c->device >= 0 && c->have_geometry) {
@@ -1054,9 +1164,13 @@ piks_status piks_set_schedule(piks_ctx *c, int32_t schedule) {
     piks_status st = cuda_check(cudaStreamSynchronize(c->stream), "schedule sync");
     if (st) return st;
   }
-  build_tiles(c);
+  c->tiles = TileJobs{};
+  c->use_tiles = false;
+  c->use_wave = wave && build_wave(c);
+  if (!c->use_wave) build_tiles(c);
   if (c->device >= 0 && c->have_geometry) {
-    piks_status st = upload_tiles(c);
+    piks_status st = upload_wave(c);
+    if (!st) st = upload_tiles(c);
     if (!st) st = cuda_check(cudaStreamSynchronize(c->stream), "schedule upload");
     if (st) return st;
     c->version += 1;
@@ -1066,7 +1180,8 @@ piks_status piks_set_schedule(piks_ctx *c, int32_t schedule) {
 
 piks_status piks_get_schedule(piks_ctx *c, int32_t *out, int32_t n) {
   if (!c || !out) return fail(PIKS_ERR_ARG, "null argument");
-  const int32_t v[7] = {c->use_tiles ? 1 : 0, c->tiles.TX, c->tiles.TY, c->tiles.TZ, c->tiles.max_rows,
+  ensure_tiles(c);
+  const int32_t v[7] = {c->use_tiles || c->use_wave ? 1 : 0, c->tiles.TX, c->tiles.TY, c->tiles.TZ, c->tiles.max_rows,
                         c->schedule, (int32_t)c->tiles.row_count.size()};
   for (int i = 0; i < n && i < 7; ++i) out[i] = v[i];
   return PIKS_OK;
@@ -1088,6 +1203,18 @@ piks_status piks_autotune(piks_ctx *c, const int32_t *cand, int32_t ncand, int32
   cudaEventCreate(&e1);
   const bool timing = c->timing;
   c->timing = false;
+  // makes candidate k the context's schedule (a column candidate ignores its tile shape)
+  auto take = [c](const int32_t *k, bool *ok) -> piks_status {
+    c->tile_dims[0] = k[0]; c->tile_dims[1] = k[1]; c->tile_dims[2] = k[2];
+    c->schedule = k[3];
+    c->tiles = TileJobs{};
+    c->use_tiles = false;
+    c->use_wave = k[3] == PIKS_SCHED_WAVE && build_wave(c);
+    *ok = c->use_wave || (k[3] != PIKS_SCHED_WAVE && build_tiles(c));
+    if (!*ok) return PIKS_OK;
+    const piks_status st = upload_wave(c);
+    return st ? st : upload_tiles(c);
+  };
   double best = 1e300;
   int bi = -1;
   piks_status st = PIKS_OK;
@@ -1096,11 +1223,10 @@ piks_status piks_autotune(piks_ctx *c, const int32_t *cand, int32_t ncand, int32
     const int32_t *k = cand + 4 * i;
     if (ms_out) ms_out[i] = -1.0;
     if (k[0] < 2 || k[1] < 2 || k[2] < 2 || (int64_t)k[0] * k[1] * k[2] > 65535) continue;
-    if (k[3] < PIKS_SCHED_TILE_DATAFLOW || k[3] > PIKS_SCHED_TILE_PIPELINED) continue;
-    c->tile_dims[0] = k[0]; c->tile_dims[1] = k[1]; c->tile_dims[2] = k[2];
-    c->schedule = k[3];
-    if (!build_tiles(c)) continue;
-    if ((st = upload_tiles(c))) break;
+    if (k[3] < PIKS_SCHED_TILE_DATAFLOW || k[3] > PIKS_SCHED_WAVE) continue;
+    bool ok = false;
+    if ((st = take(k, &ok))) break;
+    if (!ok) continue;
     enqueue_sweep(c, c->stream, epoch++);  // warm-up
     cudaEventRecord(e0, c->stream);
     for (int r = 0; r < sweeps; ++r) enqueue_sweep(c, c->stream, epoch++);
@@ -1119,10 +1245,8 @@ piks_status piks_autotune(piks_ctx *c, const int32_t *cand, int32_t ncand, int32
   if (st) return st;
   if (bi < 0) return fail(PIKS_ERR_ARG, "no usable tile candidate");
   const int32_t *k = cand + 4 * bi;
-  c->tile_dims[0] = k[0]; c->tile_dims[1] = k[1]; c->tile_dims[2] = k[2];
-  c->schedule = k[3];
-  build_tiles(c);
-  if ((st = upload_tiles(c))) return st;
+  bool ok = false;
+  if ((st = take(k, &ok))) return st;
   c->tiles_tuned = true;
   // the trial sweeps changed f: back to the state of setupFlow (all zero)
   const StateSizes z = state_sizes(c);
@@ -1201,6 +1325,12 @@ piks_status piks_geometry_array(piks_ctx *c, const char *name, void *out, int64_
   ARR("flux_list", g.flux_list) ARR("tasks", g.tasks) ARR("hyper_start", g.hyper_start) ARR("cx", c->vel.cx) ARR("cy", c->vel.cy) ARR("cz", c->vel.cz) ARR("w", c->vel.w)
   ARR("halo_send_w", g.halo_send[0]) ARR("halo_send_e", g.halo_send[1])
   ARR("halo_recv_w", g.halo_recv[0]) ARR("halo_recv_e", g.halo_recv[1])
+  if (nm.compare(0, 5, "tile_") == 0) ensure_tiles(c);
+  const WaveJobs &wj = c->wave;
+  ARR("wave_rows", wj.rows) ARR("wave_tasks", wj.tasks) ARR("wave_batch", wj.batch) ARR("wave_cols", wj.cols)
+  ARR("wave_col_list", wj.col_list)
+  int32_t waveinfo[6] = {wj.A, wj.B, wj.ring, wj.task_ring, wj.win_rows, wj.max_rows};
+  if (nm == "wave_info") { src = waveinfo; n = 6; esz = sizeof(int32_t); }
   const TileJobs &tj = c->tiles;
   ARR("tile_rows", tj.rows) ARR("tile_row_begin", tj.row_begin) ARR("tile_row_count", tj.row_count)
   ARR("tile_tasks", tj.tasks)
@@ -1482,7 +1612,9 @@ piks_status piks_launches_per_iteration(piks_ctx *c, int64_t *n) {
   if (!c || !n || !c->have_geometry) return fail(PIKS_ERR_STATE, "no geometry");
   const DevState &s = c->ds;
   int64_t k = 0;
-  if (c->use_tiles) {
+  if (c->use_wave) {
+    k += 1;
+  } else if (c->use_tiles) {
     k += (c->schedule == PIKS_SCHED_TILE_DATAFLOW || c->tiles.split) ? 1 : (int64_t)(c->tiles.launches.size() / 4);
   } else {
     for (size_t h = 0; h + 1 < c->geo.hyper_start.size(); ++h) k += c->geo.hyper_start[h + 1] > c->geo.hyper_start[h];
@@ -1495,7 +1627,15 @@ piks_status piks_launches_per_iteration(piks_ctx *c, int64_t *n) {
 
 piks_status piks_selftest_wait_timeout(piks_ctx *c, double *seconds) {
   if (!c || !seconds) return fail(PIKS_ERR_ARG, "null argument");
-  if (c->device < 0 || !c->have_geometry || !c->use_tiles || c->ds.tv.njobs < 1 || c->tiles.split)
+  if (c->device >= 0 && c->have_geometry && c->use_wave && c->ds.tv.njobs < 1) {
+    // a context that iterates the columns runs the self-test on its tile jobs
+    cudaSetDevice(c->device);
+    ensure_tiles(c);
+    piks_status st = upload_tiles(c);
+    if (!st) st = cuda_check(cudaStreamSynchronize(c->stream), "selftest tiles");
+    if (st) return st;
+  }
+  if (c->device < 0 || !c->have_geometry || !(c->use_tiles || c->use_wave) || c->ds.tv.njobs < 1 || c->tiles.split)
     return fail(PIKS_ERR_STATE, "the wait self-test needs a device state with a dataflow or diagonal tile schedule");
   cudaSetDevice(c->device);
   DevState &s = c->ds;

@@ -37,9 +37,13 @@ struct piks_ctx {
   piks::TileJobs tiles_next;
   int tiles_next_dims[3] = {0, 0, 0};
   std::future<bool> tiles_next_ready;
-  piks::TileJobs tiles;
+  piks::TileJobs tiles;             // (with the wave schedule in use: built when asked for)
   bool use_tiles = false;           // tile schedule built and uploaded
-  int schedule = PIKS_SCHED_TILE_DIAGONALS;
+  piks::WaveJobs wave;
+  bool use_wave = false;            // hyperplane-column schedule built and uploaded
+  int4 *wave_items[2] = {nullptr, nullptr};  // its items by precision (their velocity chunks differ)
+  int schedule = PIKS_SCHED_WAVE;
+  bool schedule_explicit = false;   // set by piks_set_schedule
   int prep = PIKS_PREP_DEVICE;      // where voxels are classified (device contexts)
   double setup_seconds[4] = {0, 0, 0, 0};  // last setup: box, classification, rest of the geometry, all
   int iStep = 0;

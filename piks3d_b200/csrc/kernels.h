@@ -29,6 +29,22 @@ struct TileView {
   float mean_region;
 };
 
+// Device copy of the hyperplane-column schedule (WaveJobs in piks_internal.h).
+struct WaveView {
+  const int32_t *rows;          // row codes, each batch's padded to a multiple of 4
+  const int4 *tasks;            // records as TileView::tasks, slots in the column's ring
+  const int4 *batch;            // row group (of 4), first task, rows | tasks << 16, own + static rows | ring slot << 16
+  const int4 *cols;             // [ncol][2]: first batch, batches, octant, first local hyperplane | upwind columns in x, y (or -1)
+  const int4 *items;            // (0, column, chunk, 0) in dependency order
+  int *progress;                // [ncol][nchunk] hyperplanes done, cleared before each sweep
+  int *counter;                 // item counter, cleared with the progress array behind it
+  int *err;                     // set when a wait gave up
+  int ncol, nchunk, A, B;       // columns, velocity chunks, cross-section of a column
+  int ring, task_ring, max_rows;  // ring rows, task records in flight, rows in the largest list of a group
+};
+// Shared-memory sizes of a wave launch (the largest of its members).
+struct WaveRings { int ring, task_ring, max_rows; };
+
 // Everything the kernels read, as device pointers (one struct passed by value).
 struct DevState {
   int Nx, Ny, Nz, GX, GXY;      // interior extents; ghosted row / plane strides
@@ -78,6 +94,7 @@ struct DevState {
   float *ghostW32[2], *ghostE32[2];
   const float *vtab32;          // [Nc8][kVtab] sweep constants rounded to FP32
   TileView tv;                  // tile-wavefront sweep schedule (when built)
+  WaveView wv;                  // hyperplane-column sweep schedule (when built)
   // x halos of a slab (side 0 west, 1 east; solver.F90:535-560): the nodes whose rows are
   // sent and the ghost-plane nodes received into, and per precision the send buffers (by
   // iteration parity) and the receive buffer, [count][4][Nc8] of the four octants the
@@ -141,6 +158,16 @@ void launch_tile_sweep_columns(const DevState &s, bool fp32, int epoch, cudaStre
 // Pipelined dataflow sweep over the split form: the same persistent producer / consumer
 // kernel, with single jobs in the diagonal launch order as its work items.
 void launch_tile_sweep_pipelined(const DevState &s, bool fp32, int epoch, cudaStream_t st);
+// Hyperplane-column sweep: one persistent launch per sweep (its progress array is cleared on
+// the stream first). wave_velocities() is the chunk width for a precision, wave_max_ring()
+// the ring rows that fit one CTA's shared memory beside the given task ring and row lists.
+int wave_velocities(int Nc8, bool fp32);
+int wave_max_ring(int Nc8, bool fp32, int task_ring, int max_rows);
+void launch_wave_sweep(const DevState &s, bool fp32, cudaStream_t st);
+// The same over several solves of one precision and chunk width: items (member, column, chunk,
+// 0) in dependency order; the counter and the members' progress arrays must be zero.
+void launch_wave_sweep_batch(const DevState *states, const int4 *items, int nitems, bool fp32, int V, const WaveRings &r,
+                             int *counter, int *err, cudaStream_t st);
 // Whether the column-march kernel's shared memory holds the schedule's largest job.
 bool column_sweep_fits(const TileView &tv, int Nc8, bool fp32);
 // Halo rows of iteration parity `cap`: pack the rows this slab sends into its send buffers,

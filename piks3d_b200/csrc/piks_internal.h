@@ -1,6 +1,7 @@
 // Internal host-side structures of libpiks3d_b200 (not part of the C ABI).
 #pragma once
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <new>
 #include <string>
@@ -222,6 +223,37 @@ void plan_tile_launches(TileJobs &tj, int max_classes, double ratio, bool pairs)
 // The launch plan of a precision: job pairs for the FP64 sweep (when a pair fits the shared
 // memory one job may use), single jobs for FP32 (prec: PIKS_PREC_FP64 or PIKS_PREC_FP32).
 void plan_for_precision(TileJobs &tj, int prec);
+
+// Hyperplane-column form of the sweep tasks. A column is one octant's swept nodes in an A x B
+// cross-section of the octant's frame (u, v from the inflow planes), over the whole z extent.
+// Its batches are its hyperplanes u + v + w in order: the tasks of a batch are independent of
+// one another, and a row is read only by the two batches after its own hyperplane (the scheme
+// reaches one and two cells upwind along an axis). Empty batches make their number a multiple
+// of kWaveGroup. A batch lists its own rows, then the static
+// rows (solid, corner and inflow-plane rows, never written by the sweep), then the dependent
+// rows (swept by the column upwind in x or y) that its tasks are the first to read. The rows
+// of a column's batches follow one another in a ring of `ring` shared-memory rows, at least
+// three batches' worth; slot = 1 + position modulo the ring, slot 0 is a row of zeros.
+constexpr int kWaveGroup = 4;
+struct WaveJobs {
+  int A = 0, B = 0;
+  int ncol = 0;
+  BigVec<int32_t> rows;              // rows node * 8 + octant, then (after all nodes) corner * 8 + octant of fw;
+                                     // each batch padded to a multiple of 4
+  BigVec<int32_t> tasks;             // 4 int32 per task, as TileJobs::tasks with ring slots
+  std::vector<int32_t> batch;        // 4 per batch: row list / 4, first task, rows | tasks << 16,
+                                     // own and static rows | slot of the first row << 16
+  std::vector<int32_t> cols;         // 8 per column: first batch, batches, octant, local hyperplane of the
+                                     // first batch, columns upwind in x and y or -1, 0, 0
+  std::vector<int32_t> col_list, diag;  // columns in dependency order, and their column diagonal
+  int ring = 0;                      // ring rows
+  int win_rows = 0, max_rows = 0;    // most rows in three batches in a row; rows in the largest list of a group
+  int task_ring = 0;                 // task records in flight: three groups of the largest batches
+};
+// Builds the columns from g.tasks. ring(task_ring, max_rows) gives the rows of the ring beside
+// them (0: none); false when three batches of a column need more.
+bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(int task_ring, int max_rows)> &ring,
+                     WaveJobs &wj);
 
 piks_status make_setup(const piks_params &p, Setup &s, std::string &err);
 piks_status make_velocity(const piks_params &p, Velocity &v, std::string &err);

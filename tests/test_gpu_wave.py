@@ -1,0 +1,57 @@
+"""GPU test of the hyperplane-column sweep (csrc/sweep_wave.cu, the default schedule) against the
+other schedules, bit for bit: boxes narrower than a column, boxes that end inside one and span
+several, octants of 8, 64 and 216 velocities (216: a short last chunk of velocities). FP64 against the
+per-node hyperplanes (which equal the oracle), FP32 against the tile diagonals, whose update
+is the same operations (tolerance 0 in both)."""
+import numpy as np
+import pytest
+
+import piks3d_b200 as pk
+from conftest import base_params
+from piks3d_b200 import images
+
+pytestmark = pytest.mark.gpu
+
+BOXES = [((4, 5, 6), 0.7), ((11, 10, 9), 0.5), ((12, 13, 40), 0.5), ((27, 8, 23), 0.4), ((21, 22, 5), 0.85)]
+
+
+@pytest.mark.parametrize("prec", [pk.PREC_FP64, pk.PREC_FP32])
+@pytest.mark.parametrize("nf", [2, 4, 6])
+@pytest.mark.parametrize("box,porosity", BOXES)
+def test_columns_equal_the_other_schedules(box, porosity, nf, prec):
+    nx, ny, nz = box
+    img = images.sphere_pack(max(box), porosity, 1.2, 3.0, seed=11)[:nz, :ny, :nx]
+    p = base_params(max(box), Nx=nx, Ny=ny, Nz=nz, Nc_fundamental=nf, Kn=0.6, wallExtOrder=1, fluidlayer=1)
+    out = []
+    for wave in (True, False):
+        with pk.Solver(p, device=0) as s:
+            s.set_precision(prec)
+            if wave:
+                s.setup_physical_grid(img)
+                assert s.schedule()["launch"] == pk.SCHED_WAVE
+            else:
+                s.set_tiles(*((0, 0, 0) if prec == pk.PREC_FP64 else (4, 4, 4)))
+                s.setup_physical_grid(img)
+            s.iterate(5)
+            out.append((s.get_f()[0], s.chk_converge()))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+def test_switching_schedules_keeps_the_iteration():
+    """A context that moves between the columns and the tile schedules between iterations, and
+    switches precision on the way, gives the values of one that does not."""
+    img = images.sphere_pack(18, 0.5, 1.5, 3.5, seed=2)
+    p = base_params(18, Nc_fundamental=4, Kn=0.5, wallExtOrder=1)
+    out = []
+    for moves in (True, False):
+        with pk.Solver(p, device=0) as s:
+            s.set_precision(pk.PREC_FP32)
+            s.setup_physical_grid(img)
+            for sched in (pk.SCHED_TILE_DATAFLOW, pk.SCHED_WAVE, pk.SCHED_TILE_COLUMNS, pk.SCHED_WAVE):
+                if moves:
+                    s.set_schedule(sched)
+                s.iterate(4)
+                if sched == pk.SCHED_TILE_COLUMNS:
+                    s.set_precision(pk.PREC_FP64)
+            out.append((s.get_f()[0], s.chk_converge()))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]

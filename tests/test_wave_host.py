@@ -1,0 +1,96 @@
+"""CPU test of the hyperplane-column sweep schedule (csrc/wave.cpp): the schedule is replayed in
+numpy as the kernel runs it - rows copied into a ring of exactly its size as soon as the ring's
+rule allows (overwriting what it overwrites), tasks reading ring slots only, columns one after
+another in their listed order - and every swept row must equal the per-node task list's result
+bit for bit."""
+import numpy as np
+import pytest
+
+import piks3d_b200 as pk
+from conftest import base_params
+from piks3d_b200 import images
+
+FW = 1 << 30
+
+
+def _update(own, reads, flags):
+    """A stand-in for the update that depends on every operand and its place."""
+    c = (0.31, -0.07, 0.23, -0.05, 0.19, -0.03)
+    out = 0.4 * own + 0.01
+    for k, r in enumerate(reads):
+        out = out + c[k] * r
+    return out * (1.0 + 0.125 * (flags & 1) + 0.25 * (flags >> 1 & 1) + 0.375 * (flags >> 2 & 1))
+
+
+def _replay(s, f):
+    A, B, R, task_ring, win, max_rows = s.geometry_array("wave_info").tolist()
+    rows, tasks = s.geometry_array("wave_rows"), s.geometry_array("wave_tasks").reshape(-1, 4)
+    batch, cols = s.geometry_array("wave_batch").reshape(-1, 4), s.geometry_array("wave_cols").reshape(-1, 8)
+    order = s.geometry_array("wave_col_list")
+    assert win <= R and sorted(order.tolist()) == list(range(len(cols)))
+    finished = set()
+    for col in order.tolist():
+        b0, nb, octant, s0, upx, upy = cols[col, :6].tolist()
+        for up in (upx, upy):
+            assert up < 0 or up in finished      # every upwind column comes first
+        ring = np.full(R + 1, np.nan)
+        ring[0] = 0.0
+        assert nb % 4 == 0                       # batches are requested in groups of four
+        for g in range(b0, b0 + nb, 4):
+            assert sum(-(-(int(b[2]) & 0xFFFF) // 4) * 4 for b in batch[g:g + 4]) <= max_rows
+            assert all(batch[g + i + 1, 0] == batch[g + i, 0] + -(-(int(batch[g + i, 2]) & 0xFFFF) // 4) and
+                       batch[g + i + 1, 1] == batch[g + i, 1] + (int(batch[g + i, 2]) >> 16) for i in range(3))
+        sizes = [int(b[2]) & 0xFFFF for b in batch[b0:b0 + nb]]
+        slots0 = [(int(b[3]) >> 16) & 0xFFFF for b in batch[b0:b0 + nb]]
+        start, pos = [], 0                       # ring positions without wrapping
+        for n, slot0 in zip(sizes, slots0):
+            assert slot0 == 1 + pos % R
+            start.append(pos)
+            pos += n
+        staged = 0
+        for k in range(nb):
+            # stage every batch the rule allows: batch j may go in once it overwrites nothing
+            # that batches from k - 2 on (none after k - 1 is complete) read
+            while staged < nb and start[staged] + sizes[staged] - start[max(0, k - 2)] <= R:
+                x, t0, z, w = (int(v) for v in batch[b0 + staged])
+                n, nt = z & 0xFFFF, (z >> 16) & 0xFFFF
+                assert 4 * nt <= task_ring
+                ring[1 + (start[staged] + np.arange(n)) % R] = f[rows[4 * x:4 * x + n]]
+                staged += 1
+            assert staged > k                    # three batches always fit
+            x, t0, z, w = (int(v) for v in batch[b0 + k])
+            nt, slot0 = (z >> 16) & 0xFFFF, (w >> 16) & 0xFFFF
+            new = []
+            for t in range(nt):
+                rec = tasks[t0 + t].astype(np.int64) & 0xFFFFFFFF
+                node, fl = int(rec[0]) & ((1 << 27) - 1), int(rec[0]) >> 27
+                assert int(rows[4 * x + t]) == node * 8 + octant
+                slots = [int(v) for q in rec[1:] for v in (q & 0xFFFF, q >> 16)]
+                slot = slot0 + t - (R if slot0 + t > R else 0)
+                new.append((slot, node * 8 + octant, _update(ring[slot], ring[slots], fl)))
+            for slot, row, v in new:
+                ring[slot] = v
+                f[row] = v
+        finished.add(col)
+    return f
+
+
+@pytest.mark.parametrize("n,kw", [((14, 14, 14), {}), ((21, 9, 17), dict(fluidlayer=2)), ((9, 30, 8), dict(Nc_fundamental=4)),
+                                  ((33, 19, 12), dict(block_repy=2))])
+def test_columns_replay_the_per_node_tasks(n, kw):
+    nx, ny, nz = n
+    m = max(n)
+    img = np.ascontiguousarray(images.sphere_pack(m, 0.5, 1.2, 3.5, seed=17)[:nz, :ny, :nx])
+    s = pk.Solver(base_params(m, Nx=nx, Ny=ny, Nz=nz, **kw), device=-1)
+    s.setup_physical_grid(img)
+    nn, nc = s.info()["nNodes"], s.info()["nCorner"]
+    half = 8 * nn                                # the corner rows follow the nodes' rows
+    start = np.random.default_rng(3).standard_normal(half + 8 * nc)
+    want = start.copy()
+    for t in s.geometry_array("tasks").reshape(-1, 8).tolist():
+        reads = [0.0 if c < 0 else want[(c & ~FW) + (half if c & FW else 0)] for c in t[2:]]
+        row = t[0] * 8 + (t[1] & 7)
+        want[row] = _update(want[row], reads, t[1] >> 3)
+    got = _replay(s, start.copy())
+    assert np.array_equal(got, want)
+    s.close()
