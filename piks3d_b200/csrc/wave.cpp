@@ -34,6 +34,8 @@ struct ColumnScan {
   // variant: 0 the octant's own slot, 1 / 2 what a y / z reader finds in a wall
   std::vector<Held> cell;
   std::vector<int32_t> stat, dep;
+  std::vector<int32_t> refs;      // the six reads of each task of a batch: back << 30 | list << 28 | index, -1 none
+  std::vector<int32_t> rows;      // the row lists of the worker's columns
   int32_t own[4], ns[4];          // own rows and static rows of the last four batches
   int64_t pos[4];                 // ring position of their first row
   int32_t stamp = 0;              // batches scanned so far, over all columns
@@ -41,7 +43,6 @@ struct ColumnScan {
 
 }  // namespace
 
-// One column: `fill` writes its rows and records, otherwise only the batch sizes.
 struct WaveBuilder {
   const Geometry &g;
   WaveJobs &wj;
@@ -51,103 +52,134 @@ struct WaveBuilder {
   BigVec<int32_t> order;
   std::vector<int32_t> col_of_key, key_of_col;
   std::vector<int64_t> task_begin;
+  std::vector<ColumnScan> scratch;             // by worker
+  std::vector<std::pair<int32_t, int64_t>> rows_at;  // worker and offset of each column's row list
 
-  void scan(int col, ColumnScan &c, bool fill) {
+  // One column's batches, row list and records. The ring's size is not known yet: a record
+  // holds the distance of a read's row from the first row two batches back, plus one.
+  void scan(int col, int worker) {
+    ColumnScan &c = scratch[(size_t)worker];
     const int A = wj.A, B = wj.B;
     const int key = key_of_col[(size_t)col];
     const int o = key / (ncu * ncv), ka = key % ncu, kb = key / ncu % ncv;
-    const int sx = oct_sx(o) < 0, sy = oct_sy(o) < 0, sz = oct_sz(o) < 0;
-    const int64_t t0 = task_begin[(size_t)col], t1 = task_begin[(size_t)col + 1];
+    const int32_t *tu = ux[oct_sx(o) < 0].data(), *tv = vy[oct_sy(o) < 0].data(), *tw = wz[oct_sz(o) < 0].data();
+    const int u0 = 1 + ka * A, v0 = 1 + kb * B;
+    const int64_t t1 = task_begin[(size_t)col + 1];
     int32_t *hdr = &wj.cols[(size_t)col * 8];
     const int s_first = hdr[3];
-    int64_t batch = hdr[0];
-    int64_t row_off = 0, p = t0, pos = 0;  // pos: rows of the column so far
+    int64_t batch = hdr[0], p = task_begin[(size_t)col], pos = 0;  // pos: rows of the column so far
     const int stride_v = A + 2, stride_w = (A + 2) * (B + 2);
-    auto local = [&](int32_t node, int &lu, int &lv, int &w) {
-      const uint64_t q = xyz[(size_t)node];
-      lu = ux[sx][(size_t)(q & 0x1FFFFF)] - 1 - ka * A;
-      lv = vy[sy][(size_t)((q >> 21) & 0x1FFFFF)] - 1 - kb * B;
-      w = wz[sz][(size_t)(q >> 42)];
-    };
     const int32_t first_stamp = c.stamp + 1;
+    const int64_t row0 = (int64_t)c.rows.size();
+    rows_at[(size_t)col] = {worker, row0};
+    auto where = [&](int32_t node, int &lu, int &lv, int &w) {
+      const uint64_t q = xyz[(size_t)node];
+      lu = tu[q & 0x1FFFFF] - u0;
+      lv = tv[(q >> 21) & 0x1FFFFF] - v0;
+      w = tw[q >> 42];
+    };
+    const int32_t fw0 = (int32_t)(g.node_g.size() * 8);
     for (int s = s_first; s < s_first + hdr[1]; ++s, ++batch) {
       const int32_t k = ++c.stamp;
       int64_t e = p;
+      const int64_t list0 = (int64_t)c.rows.size();
       for (; e < t1; ++e) {
         int lu, lv, w;
         const int32_t *r = &g.tasks[(size_t)order[(size_t)e] * 8];
-        local(r[0], lu, lv, w);
+        where(r[0], lu, lv, w);
         if (lu + lv + w - 1 != s) break;
-        c.cell[(size_t)(((w & 3) * stride_w + (lv + 2) * stride_v + lu + 2) * 3)] = {r[0] * 8 + o, k, (int32_t)(e - p)};
+        const int32_t code = r[0] * 8 + o;
+        c.cell[(size_t)(((w & 3) * stride_w + (lv + 2) * stride_v + lu + 2) * 3)] = {code, k, (int32_t)(e - p)};
+        c.rows.push_back(code);
       }
       const int32_t nt = (int32_t)(e - p);
       c.stat.clear();
       c.dep.clear();
-      // the row of a read: found in the column's last batches, or added to this one
-      auto find = [&](int32_t code, int axis, int back, int lu, int lv, int w) -> const Held & {
-        int cu = lu, cv = lv, cw = w;
-        (axis == 0 ? cu : axis == 1 ? cv : cw) -= back;
-        const bool fw = code & kFw;
-        const int variant = !fw && (code & 7) == o ? 0 : axis;
-        Held &h = c.cell[(size_t)(((cw & 3) * stride_w + (cv + 2) * stride_v + cu + 2) * 3 + variant)];
-        if (h.code == code && h.batch >= first_stamp && h.batch >= k - 2) return h;
-        // swept by an upwind column: a fluid node of this octant past the inflow plane
-        const bool swept = !fw && (code >> 3) < g.NF &&
-                           (axis == 0 ? ka * A + cu >= 0 : axis == 1 ? kb * B + cv >= 0 : cw >= 1);
-        std::vector<int32_t> &list = swept ? c.dep : c.stat;
-        h = {code, k, (int32_t)list.size() | (swept ? 2 : 1) << 28};
-        list.push_back(code);
-        return h;
-      };
+      c.refs.resize((size_t)nt * 6);
       for (int64_t q = p; q < e; ++q) {
         const int32_t *r = &g.tasks[(size_t)order[(size_t)q] * 8];
+        int32_t *ref = &c.refs[(size_t)(q - p) * 6];
         int lu, lv, w;
-        local(r[0], lu, lv, w);
-        for (int j = 0; j < 6; ++j)
-          if (r[2 + j] >= 0) find(r[2 + j], j >> 1, 1 + (j & 1), lu, lv, w);
+        where(r[0], lu, lv, w);
+        for (int j = 0; j < 6; ++j) {
+          const int32_t code = r[2 + j];
+          if (code < 0) { ref[j] = -1; continue; }
+          // the row of the read: one the column's last batches hold, or a new one of this batch
+          const int axis = j >> 1, back = 1 + (j & 1);
+          const int cu = axis == 0 ? lu - back : lu, cv = axis == 1 ? lv - back : lv, cw = axis == 2 ? w - back : w;
+          const bool fw = code & kFw;
+          const int variant = !fw && (code & 7) == o ? 0 : axis;
+          Held &h = c.cell[(size_t)(((cw & 3) * stride_w + (cv + 2) * stride_v + cu + 2) * 3 + variant)];
+          if (h.code != code || h.batch < first_stamp || h.batch < k - 2) {
+            // swept by an upwind column: a fluid node of this octant past the inflow plane
+            const bool swept = !fw && (code >> 3) < g.NF &&
+                               (axis == 0 ? u0 + cu >= 1 : axis == 1 ? v0 + cv >= 1 : cw >= 1);
+            std::vector<int32_t> &list = swept ? c.dep : c.stat;
+            h = {code, k, (int32_t)list.size() | (swept ? 2 : 1) << 28};
+            list.push_back(fw ? fw0 + (code & ~kFw) : code);
+          }
+          ref[j] = (int32_t)((uint32_t)(k - h.batch) << 30 | (uint32_t)h.idx);
+        }
       }
       const int32_t ns = (int32_t)c.stat.size(), nd = (int32_t)c.dep.size(), nrows = nt + ns + nd;
+      c.rows.insert(c.rows.end(), c.stat.begin(), c.stat.end());
+      c.rows.insert(c.rows.end(), c.dep.begin(), c.dep.end());
+      c.rows.resize((size_t)(list0 + (nrows + 3) / 4 * 4), 0);
       int32_t *b = &wj.batch[(size_t)batch * 4];
-      if (!fill) {
-        b[2] = nrows | nt << 16;
-        b[3] = nt + ns;
-        row_off += (nrows + 3) / 4 * 4;
-        p = e;
-        continue;
-      }
+      b[2] = nrows | nt << 16;
+      b[3] = nt + ns;
       c.own[k & 3] = nt;
       c.ns[k & 3] = ns;
       c.pos[k & 3] = pos;
-      const int R = wj.ring;
-      b[3] |= (int32_t)(1 + pos % R) << 16;
-      int32_t *rows = &wj.rows[(size_t)b[0] * 4];
-      auto slot = [&](const Held &h) -> int32_t {
-        const int list = h.idx >> 28, m = h.batch & 3;
-        const int64_t at = c.pos[m] + (h.idx & 0xFFFFFFF) + (list > 0 ? c.own[m] : 0) + (list > 1 ? c.ns[m] : 0);
-        return (int32_t)(1 + at % R);
-      };
+      int32_t from[3][3];  // by batches back and list: 1 + the position of its first row past the base
+      const int64_t base = c.pos[std::max(first_stamp, k - 2) & 3];
+      for (int back = 0; back < 3 && k - back >= first_stamp; ++back) {
+        const int m = (k - back) & 3;
+        from[back][0] = (int32_t)(1 + c.pos[m] - base);
+        from[back][1] = from[back][0] + c.own[m];
+        from[back][2] = from[back][1] + c.ns[m];
+      }
       for (int64_t q = p; q < e; ++q) {
-        const int32_t *r = &g.tasks[(size_t)order[(size_t)q] * 8];
-        rows[q - p] = r[0] * 8 + o;
-        int lu, lv, w;
-        local(r[0], lu, lv, w);
-        int32_t sl[6];
-        for (int j = 0; j < 6; ++j) sl[j] = r[2 + j] < 0 ? 0 : slot(find(r[2 + j], j >> 1, 1 + (j & 1), lu, lv, w));
+        const int32_t *r = &g.tasks[(size_t)order[(size_t)q] * 8], *ref = &c.refs[(size_t)(q - p) * 6];
+        uint32_t sl[6];
+        for (int j = 0; j < 6; ++j) {
+          const uint32_t v = (uint32_t)ref[j];
+          sl[j] = ref[j] == -1 ? 0u : (uint32_t)from[v >> 30][v >> 28 & 3] + (v & 0xFFFFFFF);
+        }
         const int fl = r[1];
         int32_t *tr = &wj.tasks[(size_t)q * 4];
         tr[0] = r[0] | ((fl & 8) ? 1 << 27 : 0) | ((fl & 16) ? 1 << 28 : 0) | ((fl & 32) ? 1 << 29 : 0);
-        tr[1] = sl[0] | sl[1] << 16;
-        tr[2] = sl[2] | sl[3] << 16;
-        tr[3] = sl[4] | sl[5] << 16;
+        for (int j = 0; j < 3; ++j) tr[1 + j] = (int32_t)(sl[2 * j] | sl[2 * j + 1] << 16);
       }
-      const int32_t fw0 = (int32_t)(g.node_g.size() * 8);
-      for (int32_t i = 0; i < ns; ++i) rows[nt + i] = c.stat[(size_t)i] & kFw ? fw0 + (c.stat[(size_t)i] & ~kFw) : c.stat[(size_t)i];
-      std::copy(c.dep.begin(), c.dep.end(), rows + nt + ns);
-      std::fill(rows + nrows, rows + (nrows + 3) / 4 * 4, 0);
       pos += nrows;
       p = e;
     }
-    if (!fill) hdr[6] = (int32_t)(row_off / 4);  // row groups of the column (an offset later)
+    hdr[6] = (int32_t)(((int64_t)c.rows.size() - row0) / 4);  // row groups of the column (an offset later)
+  }
+
+  // The column's row list to its place, its records' distances to ring slots.
+  void place(int col) {
+    const int32_t *hdr = &wj.cols[(size_t)col * 8];
+    int32_t *b = &wj.batch[(size_t)hdr[0] * 4];
+    const auto &[worker, row0] = rows_at[(size_t)col];
+    const int32_t *rows = scratch[(size_t)worker].rows.data() + row0;
+    std::copy(rows, rows + (int64_t)hdr[6] * 4, &wj.rows[(size_t)b[0] * 4]);
+    const uint32_t R = (uint32_t)wj.ring;
+    uint32_t at = 0, start[3] = {0, 0, 0};  // positions (mod R) of the batch and the two before it
+    for (int i = 0; i < hdr[1]; ++i, b += 4) {
+      start[2] = i > 1 ? start[1] : 0; start[1] = i > 0 ? start[0] : 0; start[0] = at;
+      b[3] |= (int32_t)(1 + at) << 16;
+      int32_t *tr = &wj.tasks[(size_t)b[1] * 4];
+      const uint32_t base = start[2];
+      // a window of three batches is at most the ring: one wrap
+      auto slot = [&](uint32_t d) { return d == 0 ? 0u : base + d > R ? base + d - R : base + d; };
+      for (int32_t q = 0; q < b[2] >> 16; ++q, tr += 4)
+        for (int j = 1; j < 4; ++j) {
+          const uint32_t v = (uint32_t)tr[j];
+          tr[j] = (int32_t)(slot(v & 0xFFFF) | slot(v >> 16) << 16);
+        }
+      at = (at + (uint32_t)(b[2] & 0xFFFF)) % R;
+    }
   }
 };
 
@@ -156,8 +188,9 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   wj.A = A;
   wj.B = B;
   const int64_t ntask = (int64_t)(g.tasks.size() / 8);
-  if (ntask <= 0 || ntask > INT32_MAX || A < 2 || B < 2) return false;
-  WaveBuilder wb{g, wj, 0, 0, {}, {}, {}, {}, {}, {}, {}, {}};
+  // (the distances of a window of three batches have to fit 16 bits)
+  if (ntask <= 0 || ntask > INT32_MAX || A < 2 || B < 2 || A * B > 2048) return false;
+  WaveBuilder wb{g, wj, 0, 0, {}, {}, {}, {}, {}, {}, {}, {}, {}, {}};
   // frame coordinates: 0 on the inflow plane of the octant's sign, the swept planes from 1
   const int ux_pos = g.wglob ? 1 : g.xl - 1, ux_neg = g.eglob ? g.Nx : g.xu + 1;
   auto axis = [](int G, int at_pos, int at_neg, std::vector<int32_t> *out) {
@@ -243,15 +276,14 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   }
   if (nbatch > INT32_MAX / 4) return false;
   wj.batch.assign((size_t)nbatch * 4, 0);
-  auto each_column = [&](bool fill) {
-    std::atomic<int> next{0};
-    on_workers(nw, [&](int) {
-      ColumnScan c;
-      c.cell.assign((size_t)4 * (A + 2) * (B + 2) * 3, Held{-1, 0, 0});
-      for (int col; (col = next.fetch_add(1)) < ncol;) wb.scan(col, c, fill);
-    });
-  };
-  each_column(false);
+  wj.tasks.resize((size_t)ntask * 4);
+  wb.scratch.resize((size_t)nw);
+  wb.rows_at.resize((size_t)ncol);
+  std::atomic<int> next{0};
+  on_workers(nw, [&](int t) {
+    wb.scratch[(size_t)t].cell.assign((size_t)4 * (A + 2) * (B + 2) * 3, Held{-1, 0, 0});
+    for (int col; (col = next.fetch_add(1)) < ncol;) wb.scan(col, t);
+  });
   // windows of three batches: the rows that have to be on chip at once (a batch's rows are
   // read in the next two)
   int64_t groups = 0;
@@ -275,7 +307,6 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
       task += b[4 * i + 2] >> 16;
     }
     groups += h[6];
-    h[6] = 0;
   }
   wj.max_rows = max_rows;
   wj.win_rows = win_rows;
@@ -284,8 +315,10 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   wj.ring = std::min(ring(wj.task_ring, wj.max_rows), 65000);
   if (wj.ring < win_rows) return false;
   wj.rows.resize((size_t)groups * 4);
-  wj.tasks.resize((size_t)ntask * 4);
-  each_column(true);
+  next = 0;
+  on_workers(nw, [&](int) {
+    for (int col; (col = next.fetch_add(1)) < ncol;) wb.place(col);
+  });
   // columns in dependency order: by the x + y column diagonal of the octant's frame
   wj.col_list.resize((size_t)ncol);
   for (int i = 0; i < ncol; ++i) wj.col_list[(size_t)i] = i;
