@@ -328,7 +328,7 @@ class Solver:
         """Rho, Ux, Uy, Uz as (Nz, Ny, Nx) arrays (0 at non-fluid voxels)."""
         inf = self.info()
         shape = (inf["Nz"], inf["Ny"], inf["Nx"])
-        out = [np.zeros(shape, dtype=np.float64) for _ in range(4)]
+        out = [np.empty(shape, dtype=np.float64) for _ in range(4)]
         _check(self.lib.piks_get_macro(self._ctx, *[_dptr(a) for a in out]))
         return tuple(out)
 
