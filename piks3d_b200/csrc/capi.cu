@@ -298,9 +298,12 @@ void enqueue_boundaries_timed(piks_ctx *c, cudaStream_t st, int n) {
   {
     Timed t(c, KT_WALLS);
     const auto &ls = c->geo.level_start;
-    for (size_t L = 0; L + 1 < ls.size(); ++L) {
-      if (f32) launch_walls32(s, ls[L], ls[L + 1], prev, st);
-      else launch_walls(s, ls[L], ls[L + 1], prev, st);
+    // (walls that extrapolate from their first point only read no other wall: one launch)
+    const size_t n = ls.empty() ? 0 : s.wall_far ? ls.size() - 1 : std::min<size_t>(ls.size() - 1, 1);
+    for (size_t L = 0; L < n; ++L) {
+      const int end = s.wall_far ? ls[L + 1] : ls.back();
+      if (f32) launch_walls32(s, ls[L], end, prev, st);
+      else launch_walls(s, ls[L], end, prev, st);
     }
   }
   { Timed t(c, KT_INLET); f32 ? launch_inlet_outlet32(s, prev, st) : launch_inlet_outlet(s, prev, st); }
@@ -738,9 +741,22 @@ piks_status piks_setup_physical_grid(piks_ctx *c, const uint8_t *raw, int64_t nb
   UP(g.wall_node, wall_node, pi); UP(g.wall_label, wall_label, pi); UP(g.wall_corner, wall_corner, pi);
   UP(g.wall_nb, wall_nb, pi); UP(g.wall_order, wall_order, pi); UP(g.wall_e, wall_e, pd);
   {
-    std::vector<int32_t> rec(g.wall_order.size() * 16, 0);
-    for (size_t w = 0; w < g.wall_order.size(); ++w) {
-      const size_t q = (size_t)g.wall_order[w];
+    // wall records label by label within windows of a level (see DevState::wall_rec)
+    std::vector<int32_t> order(g.wall_order.size()), rec(g.wall_order.size() * 16, 0);
+    for (size_t L = 0; L + 1 < g.level_start.size(); ++L)
+      for (int64_t w0 = g.level_start[L], w1; w0 < g.level_start[L + 1]; w0 = w1) {
+        w1 = std::min<int64_t>(w0 + 2048, g.level_start[L + 1]);
+        int32_t at[129] = {0};  // labels are below 128
+        for (int64_t w = w0; w < w1; ++w) at[g.wall_label[(size_t)g.wall_order[(size_t)w]] + 1]++;
+        for (int v = 0; v < 128; ++v) at[v + 1] += at[v];
+        for (int64_t w = w0; w < w1; ++w) {
+          const int32_t q = g.wall_order[(size_t)w];
+          order[(size_t)(w0 + at[g.wall_label[(size_t)q]]++)] = q;
+        }
+      }
+    for (size_t w = 0; w < order.size(); ++w) {
+      const size_t q = (size_t)order[w];
+      s.wall_far |= g.wall_e[2 * q + 1] != 0.0;
       int32_t *r = &rec[w * 16];
       r[0] = g.wall_node[q]; r[1] = g.wall_corner[q]; r[2] = g.wall_label[q];
       std::memcpy(r + 4, &g.wall_e[2 * q], 2 * sizeof(double));

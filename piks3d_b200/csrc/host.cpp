@@ -47,13 +47,12 @@ const WProg *wall_program(int label) {
 
 bool make_wall_plan(const WProg &p, WPlan &out) {
   out = WPlan{};
-  out.nface = p.nface;
-  out.nwr = p.nwr;
+  out.nface = (uint32_t)p.nface;
+  out.nwr = (uint32_t)p.nwr;
   if (p.nface < 1 || p.nface > 3 || p.nwr > 12) return false;
   for (int f = 0; f < p.nface; ++f) {
-    out.dir[f] = p.face[f].dir;
-    out.store[f] = p.face[f].store;
-    out.keep[f] = p.face[f].store == ST_Z ? 0 : 0xf;
+    out.face[f] = (uint32_t)(p.face[f].dir << 12 | p.face[f].store << 15 | (p.face[f].store == ST_Z ? 0 : 0xf) << 17);
+    for (int m = 0; m < 4; ++m) out.face[f] |= (uint32_t)((kIncoming[p.face[f].dir][m] - 1) << (3 * m));
   }
   for (int k = 0; k < p.nwr; ++k) {
     const WWrite &w = p.wr[k];
@@ -71,11 +70,8 @@ bool make_wall_plan(const WProg &p, WPlan &out) {
       if (p.wr[j].dst_store == w.dst_store && p.wr[j].dst_o == w.dst_o) return false;
     for (int f = 0; f < p.nface; ++f)
       for (int m = 0; m < 4; ++m)
-        if (p.face[f].store == w.dst_store && kIncoming[p.face[f].dir][m] == w.dst_o) out.keep[f] &= ~(1 << m);
-    out.dst_store[k] = w.dst_store;
-    out.dst_o[k] = w.dst_o - 1;
-    out.face[k] = w.face;
-    out.src[k] = src;
+        if (p.face[f].store == w.dst_store && kIncoming[p.face[f].dir][m] == w.dst_o) out.face[f] &= ~(1u << (17 + m));
+    out.wr[k] = (uint32_t)(src | (w.dst_o - 1) << 4 | w.face << 8 | (w.dst_store == ST_F ? 1 : 0) << 10);
   }
   return true;
 }

@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256, 5) k_walls(const DevState a, int begin, i
   double rho0 = 0.0, rho1 = 0.0, rho2 = 0.0;
   for (int fi = 0; fi < nface; ++fi) {
     const int dir = P.face[fi].dir, st = P.face[fi].store;
-    const int n1 = nb[2 * fi], code = nb[2 * fi + 1];
+    const int n1 = nb[2 * fi], code = e2 == 0.0 ? -1 : nb[2 * fi + 1];
     const double *plane = nullptr;
     size_t prow = 0;
     if (code < -1) {
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256, 5) k_walls(const DevState a, int begin, i
         else {
           double n1v[VPL], farv[VPL];
           ld_vpl<VPL>(a.h + hidx(nb[2 * zface], so, Nc8, lf), n1v);
-          const int code = nb[2 * zface + 1];
+          const int code = e2 == 0.0 ? -1 : nb[2 * zface + 1];
 #pragma unroll
           for (int v = 0; v < VPL; ++v) farv[v] = 0.0;
           if (code >= 0) ld_vpl<VPL>(a.h + hidx(code, so, Nc8, lf), farv);
@@ -346,111 +346,131 @@ __global__ void __launch_bounds__(256, 5) k_walls(const DevState a, int begin, i
   }
 }
 
-// The diffuse wall for octants of at most 32 * VPL velocities (one pass of the warp), with
-// the extrapolated face values kept in shared memory: the re-emission reads them there
-// (WPlan) instead of re-loading the slots, and a face value is stored only where it is
-// the slot's final content. Same operations on the same operands as k_walls, in the same
-// order; per warp, 12 * Nc8 face values and Nc8 density terms. One wall (warp) per block,
-// 24 blocks per SM (74 registers, no spills): a block's shared memory is free as soon as its
-// wall is done (per iteration on a 128^3 pack: 8 walls per block 0.758 ms, 4 0.698, 2 0.648,
-// 1 0.615).
-constexpr int kWallWarps = 1;
-template <int VPL>
-__global__ void __launch_bounds__(kWallWarps * 32, 24 / kWallWarps) k_walls_onchip(const DevState a, int begin, int end, int gbuf) {
+// Shared memory of a wall in k_walls_rows, in doubles: 12 near rows (then the extrapolated
+// values), 12 far rows where some wall has an e2, 3 padded rows of density terms. Walls of a
+// warp (LPW = 4) start half a 128-byte line apart.
+__host__ __device__ constexpr int wall_doubles(int LPW, int Nc8, int far_rows) {
+  const int n = (12 + far_rows) * Nc8 + 3 * (Nc8 + 2);
+  return LPW == 32 ? n + (n & 1) : (n + 15) / 16 * 16 + 8;
+}
+
+// The diffuse wall with its rows on chip, LPW lanes per wall (32 / LPW walls per warp, or LPW / 32
+// warps per wall) and two velocities per lane. All rows of a wall are asked for at once (cp.async
+// into shared memory: a lane copies what it reads itself), then every face is extrapolated, the
+// densities are summed serially over l in the reference's order, a lane per face, and the
+// re-emission reads the extrapolated values on chip (WPlan); a face value is stored only where it
+// is the slot's final content. Same operations on the same operands as k_walls, in the same order.
+// The far point's rows are read where its coefficient is not 0 (wallExtOrder 1 makes it 0).
+// What bounds it: the rows' bytes (2.1 GB a pass on a 128^3 pack of 300,000 walls, 512
+// velocities, 0.33 ms at the copy rate) with 29 walls of 7.6 KB on an SM. A warp that took face
+// after face, each a load round trip and a serial sum, needed 0.595 ms; this needs 0.40. With 1728
+// velocities (75 x 53 x 37 pack, 20,000 walls), where the rows went through L2 twice, 0.476 -> 0.119 ms.
+template <int LPW>
+__global__ void __launch_bounds__(LPW <= 32 ? 32 : LPW, LPW <= 32 ? 26 : LPW == 128 ? 8 : 3)
+k_walls_rows(const DevState a, int begin, int end, int gbuf, int far_rows) {
   extern __shared__ __align__(16) double wall_sm[];
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int widx = begin + (int)blockIdx.x * kWallWarps + wib;
-  if (widx >= end) return;  // whole warp (only warp-level synchronisation below)
+  const int t = threadIdx.x % LPW;
+  const int widx = begin + (LPW <= 32 ? (int)blockIdx.x * (32 / LPW) + (int)threadIdx.x / LPW : (int)blockIdx.x);
+  if (widx >= end) return;  // the wall's lanes together
+  const unsigned seg = LPW >= 32 ? 0xffffffffu : (((1u << (LPW & 31)) - 1u) << (threadIdx.x & 31 & ~(LPW - 1)));
   const int Nc8 = a.Nc8;
-  double *E = wall_sm + (size_t)wib * 13 * Nc8;
-  double *Tm = E + 12 * Nc8;
-  // the wall's fields from its level-order record (one round trip; see DevState::wall_rec)
+  double *E = wall_sm + (LPW <= 32 ? (int)threadIdx.x / LPW * wall_doubles(LPW, Nc8, far_rows) : 0);
+  double *Tm = E + (12 + far_rows) * Nc8;
+  const int Ts = Nc8 + 2;
   const int4 *rp = a.wall_rec + (size_t)widx * 4;
-  const int4 r0 = __ldg(rp);
+  const int4 r0 = __ldg(rp), nb0 = __ldg(rp + 2), nb1 = __ldg(rp + 3);
   const double2 ee = __ldg(reinterpret_cast<const double2 *>(rp + 1));
-  const int node = r0.x;
-  const int corner = r0.y;
-  const WPlan &P = c_plan[c_prog_of[r0.z]];
   const double e1 = ee.x, e2 = ee.y;
-  const int nface = P.nface;
-  const int lf = lane * VPL;
+  const WPlan &P = c_plan[c_prog_of[r0.z]];
+  const int nface = (int)P.nface, lf = t * 2;
   const bool lv = lf < Nc8;
-  double rho0 = 0.0, rho1 = 0.0, rho2 = 0.0;
-  for (int fi = 0; fi < nface; ++fi) {
-    const int dir = P.dir[fi], st = P.store[fi], keep = P.keep[fi];
-    // the face's (neighbour, far point) pair: the record's second half, an L1 hit
-    const int2 nbp = __ldg(reinterpret_cast<const int2 *>(rp + 2) + fi);
-    const int n1 = nbp.x, code = nbp.y;
-    if (lv) {
-      const double *plane = nullptr;
-      size_t prow = 0;
-      if (code < -1) {
-        const int cc = -code - 2;
-        plane = (cc & 1) ? a.ghostE[gbuf] : a.ghostW[gbuf];
-        prow = (size_t)(cc >> 1) * 4;
+  if (lv) {
+    for (int fi = 0; fi < nface; ++fi) {
+      const uint32_t F = P.face[fi];
+      const int n1 = fi == 0 ? nb0.x : fi == 1 ? nb0.z : nb1.x, code = fi == 0 ? nb0.y : fi == 1 ? nb0.w : nb1.y;
+      const double *np = a.h + hidx(n1, 0, Nc8, lf);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) cp_async16_cg(E + (fi * 4 + m) * Nc8 + lf, np + (F >> (3 * m) & 7) * Nc8);
+      if (e2 == 0.0 || code == -1) continue;
+      const int cc = -code - 2;
+      const double *plane = (cc & 1) ? a.ghostE[gbuf] : a.ghostW[gbuf];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int oo = F >> (3 * m) & 7;
+        cp_async16_cg(E + (12 + fi * 4 + m) * Nc8 + lf,
+                      code >= 0 ? a.h + hidx(code, oo, Nc8, lf)
+                                : plane + ((size_t)(cc >> 1) * 4 + plane_slot(oo)) * Nc8 + lf);
       }
-      double near_[4][VPL], far_[4][VPL];
-#pragma unroll
-      for (int mm = 0; mm < 4; ++mm) {
-        const int oo = c_incoming[dir][mm] - 1;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) far_[mm][v] = 0.0;
-        ld_vpl<VPL>(a.h + hidx(n1, oo, Nc8, lf), near_[mm]);
-        if (code >= 0) ld_vpl<VPL>(a.h + hidx(code, oo, Nc8, lf), far_[mm]);
-        else if (plane) ld_vpl<VPL>(plane + (prow + plane_slot(oo)) * Nc8 + lf, far_[mm]);
-      }
-      double ext[4][VPL];
-#pragma unroll
-      for (int mm = 0; mm < 4; ++mm) {
-        const int oo = c_incoming[dir][mm] - 1;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) ext[mm][v] = dadd(dmul(e1, near_[mm][v]), dmul(e2, far_[mm][v]));
-        st_vpl<VPL>(E + (size_t)(fi * 4 + mm) * Nc8 + lf, ext[mm]);
-        if (keep >> mm & 1) {
-          if (st == ST_F) st_vpl<VPL>(a.h + hidx(node, oo, Nc8, lf), ext[mm]);
-          else st_vpl<VPL>(a.fw + hidx(corner, oo, Nc8, lf), ext[mm]);
-        }
-      }
-      double tface[VPL];
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int l = lf + v;
-        const double ca = dir < 2 ? __ldg(a.cx + l) : dir < 4 ? __ldg(a.cy + l) : __ldg(a.cz + l);
-        tface[v] = dmul(ca, dadd(dadd(dadd(ext[0][v], ext[1][v]), ext[2][v]), ext[3][v]));
-      }
-      st_vpl<VPL>(Tm + lf, tface);
     }
-    __syncwarp();
-    // rho_face = sum over l in ascending order (every lane, broadcast reads)
-    double racc = 0.0;
-    int l = 0;
-    for (; l + 8 <= Nc8; l += 8) {
-      double t[8];
+    cp_async_commit();
+    cp_async_wait<0>();
+    double *hn = a.h + hidx(r0.x, 0, Nc8, lf), *wn = a.fw + hidx(r0.y, 0, Nc8, lf);
+    for (int fi = 0; fi < nface; ++fi) {
+      const uint32_t F = P.face[fi];
+      const int dir = F >> 12 & 7, code = fi == 0 ? nb0.y : fi == 1 ? nb0.w : nb1.y;
+      const bool far = e2 != 0.0 && code != -1;
+      double *out = (F >> 15 & 3) == ST_F ? hn : wn;
+      double ext[4][2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) t[j] = Tm[l + j];
+      for (int m = 0; m < 4; ++m) {
+        double near_[2], far_[2] = {0.0, 0.0};
+        ld_vpl_sm<2>(E + (fi * 4 + m) * Nc8 + lf, near_);
+        if (far) ld_vpl_sm<2>(E + (12 + fi * 4 + m) * Nc8 + lf, far_);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) racc = dadd(racc, t[j]);
+        for (int v = 0; v < 2; ++v) ext[m][v] = dadd(dmul(e1, near_[v]), dmul(e2, far_[v]));
+        st_vpl<2>(E + (fi * 4 + m) * Nc8 + lf, ext[m]);
+        if (F >> (17 + m) & 1) st_vpl<2>(out + (F >> (3 * m) & 7) * Nc8, ext[m]);
+      }
+      double ca[2], tface[2];
+      ld_vpl_sm<2>((dir < 2 ? a.cx : dir < 4 ? a.cy : a.cz) + lf, ca);
+#pragma unroll
+      for (int v = 0; v < 2; ++v) tface[v] = dmul(ca[v], dadd(dadd(dadd(ext[0][v], ext[1][v]), ext[2][v]), ext[3][v]));
+      st_vpl<2>(Tm + fi * Ts + lf, tface);
     }
-    for (; l < Nc8; ++l) racc = dadd(racc, Tm[l]);
-    __syncwarp();  // Tm is rewritten by the next face
-    if (fi == 0) rho0 = racc; else if (fi == 1) rho1 = racc; else rho2 = racc;
+  }
+  if (LPW <= 32) __syncwarp(seg); else __syncthreads();
+  // rho_face: lane fi sums face fi's terms over l in ascending order (Nc8 is a multiple of 8)
+  double rho = 0.0;
+  if (t < nface) {
+    const double2 *T = reinterpret_cast<const double2 *>(Tm + t * Ts);
+    for (int l = 0; l < Nc8 / 2; l += 4) {
+      double2 x[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = T[l + j];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rho = dadd(dadd(rho, x[j].x), x[j].y);
+    }
+    rho = __ddiv_rn(rho, a.DiffFlux);
+  }
+  double rf[3];
+  if (LPW <= 32) {
+    const int base = threadIdx.x & 31 & ~(LPW - 1);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) rf[f] = __shfl_sync(seg, rho, base + f);
+  } else {
+    __shared__ double rho_sm[3];
+    if (t < 3) rho_sm[t] = rho;
+    __syncthreads();
+#pragma unroll
+    for (int f = 0; f < 3; ++f) rf[f] = rho_sm[f];
   }
   if (!lv) return;
-  rho0 = __ddiv_rn(rho0, a.DiffFlux);
-  if (nface > 1) rho1 = __ddiv_rn(rho1, a.DiffFlux);
-  if (nface > 2) rho2 = __ddiv_rn(rho2, a.DiffFlux);
   const double one_m = dsub(1.0, a.accom);
-  double aw[VPL];
+  double aw[2];
+  ld_vpl_sm<2>(a.w + lf, aw);
 #pragma unroll
-  for (int v = 0; v < VPL; ++v) aw[v] = dmul(a.accom, __ldg(a.w + lf + v));
-  for (int k = 0; k < P.nwr; ++k) {
-    double src[VPL], val[VPL];
-    ld_vpl_sm<VPL>(E + (size_t)P.src[k] * Nc8 + lf, src);
-    const double rf = P.face[k] == 0 ? rho0 : P.face[k] == 1 ? rho1 : rho2;
+  for (int v = 0; v < 2; ++v) aw[v] = dmul(a.accom, aw[v]);
+  double *hn = a.h + hidx(r0.x, 0, Nc8, lf), *wn = a.fw + hidx(r0.y, 0, Nc8, lf);
+  const int nwr = (int)P.nwr;
+  for (int k = 0; k < nwr; ++k) {
+    const uint32_t W = P.wr[k];
+    double src[2], val[2];
+    ld_vpl_sm<2>(E + (W & 15) * Nc8 + lf, src);
+    const int f = W >> 8 & 3;
+    const double r = f == 0 ? rf[0] : f == 1 ? rf[1] : rf[2];
 #pragma unroll
-    for (int v = 0; v < VPL; ++v) val[v] = dadd(dmul(aw[v], rf), dmul(one_m, src[v]));
-    if (P.dst_store[k] == ST_F) st_vpl<VPL>(a.h + hidx(node, P.dst_o[k], Nc8, lf), val);
-    else st_vpl<VPL>(a.fw + hidx(corner, P.dst_o[k], Nc8, lf), val);
+    for (int v = 0; v < 2; ++v) val[v] = dadd(dmul(aw[v], r), dmul(one_m, src[v]));
+    st_vpl<2>((W >> 10 & 1 ? hn : wn) + (W >> 4 & 7) * Nc8, val);
   }
 }
 
@@ -990,18 +1010,27 @@ void launch_moments(const DevState &s, cudaStream_t st) {
   k_moments<<<blocks_for((size_t)s.NF, kMomWarps * 32), kMomWarps * 32, sizeof(MomSmem), st>>>(s);
 }
 
+namespace {
+template <int LPW>
+void launch_walls_rows(const DevState &s, int begin, int end, int gbuf, cudaStream_t st) {
+  const int walls = LPW <= 32 ? 32 / LPW : 1, far_rows = s.wall_far ? 12 : 0;
+  once_per_device(reinterpret_cast<const void *>(k_walls_rows<LPW>), [](int) {
+    const int most = (int)sizeof(double) * wall_doubles(LPW, LPW == 4 ? 8 : 2 * LPW, 12) * (LPW <= 32 ? 32 / LPW : 1);
+    cudaFuncSetAttribute(k_walls_rows<LPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  });
+  const size_t smem = sizeof(double) * (size_t)wall_doubles(LPW, s.Nc8, far_rows) * walls;
+  k_walls_rows<LPW><<<(end - begin + walls - 1) / walls, LPW <= 32 ? 32 : LPW, smem, st>>>(s, begin, end, gbuf, far_rows);
+}
+}  // namespace
+
+// Octants of 8, 64, 216 and 512 velocities keep a wall's rows on chip; 1728 and more do not fit.
 void launch_walls(const DevState &s, int begin, int end, int gbuf, cudaStream_t st) {
   if (end <= begin) return;
-  if (g_plan_ok && s.Nc8 <= 64 && (s.Nc8 <= 32 || s.Nc8 % 2 == 0)) {
-    once_per_device(reinterpret_cast<const void *>(k_walls_onchip<1>), [](int) {
-      const int most = kWallWarps * 13 * 64 * (int)sizeof(double);
-      cudaFuncSetAttribute(k_walls_onchip<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      cudaFuncSetAttribute(k_walls_onchip<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    });
-    const size_t smem = (size_t)kWallWarps * 13 * s.Nc8 * sizeof(double);
-    const unsigned grid = blocks_for((size_t)(end - begin), kWallWarps);
-    if (s.Nc8 > 32) k_walls_onchip<2><<<grid, kWallWarps * 32, smem, st>>>(s, begin, end, gbuf);
-    else k_walls_onchip<1><<<grid, kWallWarps * 32, smem, st>>>(s, begin, end, gbuf);
+  if (g_plan_ok && s.Nc8 <= 512 && s.Nc8 % 8 == 0) {
+    if (s.Nc8 == 8) launch_walls_rows<4>(s, begin, end, gbuf, st);
+    else if (s.Nc8 <= 64) launch_walls_rows<32>(s, begin, end, gbuf, st);
+    else if (s.Nc8 <= 256) launch_walls_rows<128>(s, begin, end, gbuf, st);
+    else launch_walls_rows<256>(s, begin, end, gbuf, st);
     return;
   }
   const size_t threads = (size_t)(end - begin) * 32;

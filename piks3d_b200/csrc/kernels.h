@@ -69,11 +69,10 @@ struct DevState {
   const double *wall_e;
   // the same fields in level order, one 64-byte record (four int4) per wall position:
   // node, corner, label, 0 | e1, e2 (FP64) | nb[0..3] | nb[4], nb[5], 0, 0; the on-chip wall
-  // kernels read a wall's fields in one round trip instead of two (wall_order, then the
-  // rest). Per iteration on a 128^3 pack: FP32 0.476 -> 0.446 ms; FP64 0.845 -> 0.758 ms
-  // together with up to 85 registers per thread instead of 64 (no spills; the records alone at 64
-  // registers spilled and took 0.870 against 0.834)
+  // kernels read a wall's fields in one round trip. Inside a level the records stand label by
+  // label within windows of 2048 walls, so that the walls of a warp mostly share a program.
   const int4 *wall_rec;
+  int wall_far;                 // 1 when a wall extrapolates from its second point (e2 != 0)
   // post-sweep switch commits
   int ncommit;
   const int32_t *commit;

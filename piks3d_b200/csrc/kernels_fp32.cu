@@ -24,6 +24,11 @@ __device__ __forceinline__ size_t hidx(int node, int o, int Nc8, int l) {
 }
 __device__ __forceinline__ int plane_slot(int o) { return o >> 1; }
 constexpr int kFwBit = 1 << 30;
+__device__ __forceinline__ void cp_async16_cg(void *smem, const void *gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 template <int VPL>
 __device__ __forceinline__ void ld32(const float *p, float (&v)[VPL]) {
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(256) k_walls32(const DevState a, int begin, in
   const int nface = P.nface;
   const int chunkw = LANES * VPL;
   auto far_ptr = [&](int code, int oo, int lf) -> const float * {
-    if (e2 == 0.f) return nullptr;  // as in k_walls32_onchip
+    if (e2 == 0.f) return nullptr;  // as in k_walls32_rows
     if (code >= 0) return a.h32 + hidx(code, oo, Nc8, lf);
     if (code == -1) return nullptr;
     const int cc = -code - 2;
@@ -235,102 +240,121 @@ __global__ void __launch_bounds__(256) k_walls32(const DevState a, int begin, in
   }
 }
 
-// The FP32 diffuse wall for octants of at most LANES * VPL velocities (one pass of the
-// lane segment), with the extrapolated face values kept in shared memory (12 * Nc8 floats
-// per wall): the re-emission reads them there (WPlan) instead of re-loading the slots,
-// and a face value is stored only where it is the slot's final content.
-template <int VPL, int LANES>
-__global__ void __launch_bounds__(256, 3) k_walls32_onchip(const DevState a, int begin, int end, int gbuf) {
+// Shared memory of a wall in k_walls32_rows, in floats: 12 near rows (then the extrapolated
+// values) and 12 far rows where some wall has an e2; walls of 8 velocities start 32 bytes past a
+// multiple of 128, so that the four walls of a quarter-warp request use different banks.
+__host__ __device__ constexpr int wall32_floats(int Nc8, int far_rows) {
+  return (12 + far_rows) * Nc8 + (Nc8 == 8 ? 8 : 0);
+}
+
+// The FP32 diffuse wall for octants of 4 * LANES velocities, LANES lanes per wall and four
+// velocities per lane: all rows of a wall are asked for at once (cp.async into shared memory: a
+// lane copies what it reads itself), every face is extrapolated, the densities are summed in FP64
+// (four velocities in the lane, then the lanes), and the re-emission reads the extrapolated values
+// on chip (WPlan); a face value is stored only where it is the slot's final content.
+// What bounds it: the rows' bytes (1.1 GB a pass on a 128^3 pack of 300,000 walls, 512 velocities,
+// 0.165 ms at the copy rate: 0.189 ms). A version with separate plan fields, a load round trip per
+// face and mixed programs in a warp was bound by its instructions: 0.430 ms there, and 0.156 against
+// 0.023 ms on a 96^3 pack of 64 velocities, where a warp now takes 16 walls instead of 4.
+template <int LANES>
+__global__ void __launch_bounds__(64, 18) k_walls32_rows(const DevState a, int begin, int end, int gbuf, int far_rows) {
   extern __shared__ __align__(16) float wall32_sm[];
-  const int wib = threadIdx.x / LANES;
-  const int widx = begin + (int)blockIdx.x * (256 / LANES) + wib;
+  constexpr int Nc8 = LANES * 4;
+  const int widx = begin + (int)blockIdx.x * (64 / LANES) + (int)threadIdx.x / LANES;
   if (widx >= end) return;  // whole segment
-  const int lane = threadIdx.x % LANES;
-  const unsigned seg = LANES == 32 ? 0xffffffffu : (((1u << LANES) - 1u) << (threadIdx.x & 31 & ~(LANES - 1)));
-  const int Nc8 = a.Nc8;
-  float *E = wall32_sm + (size_t)wib * 12 * Nc8;
+  const int lane = threadIdx.x % LANES, lf = lane * 4;
+  const unsigned seg = ((1u << LANES) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
+  float *E = wall32_sm + (int)threadIdx.x / LANES * wall32_floats(Nc8, far_rows) + lf;
   const int4 *rp = a.wall_rec + (size_t)widx * 4;
-  const int4 r0 = __ldg(rp);
+  const int4 r0 = __ldg(rp), nb0 = __ldg(rp + 2), nb1 = __ldg(rp + 3);
   const double2 ee = __ldg(reinterpret_cast<const double2 *>(rp + 1));
-  const int node = r0.x;
-  const int corner = r0.y;
-  const WPlan &P = c32_plan[c32_prog_of[r0.z]];
   const float e1 = (float)ee.x, e2 = (float)ee.y;
-  const int nface = P.nface;
-  const int lf = lane * VPL;
-  const bool lv = lf < Nc8;
-  // the second extrapolation point only matters when its coefficient does (wallExtOrder 1
-  // makes it 0: the FP32 path, exact to its tolerance and not to the bit, skips the load)
-  auto far_ptr = [&](int code, int oo) -> const float * {
-    if (e2 == 0.f) return nullptr;
-    if (code >= 0) return a.h32 + hidx(code, oo, Nc8, lf);
-    if (code == -1) return nullptr;
+  const WPlan &P = c32_plan[c32_prog_of[r0.z]];
+  const int nface = (int)P.nface;
+  for (int fi = 0; fi < nface; ++fi) {
+    const uint32_t F = P.face[fi];
+    const int n1 = fi == 0 ? nb0.x : fi == 1 ? nb0.z : nb1.x, code = fi == 0 ? nb0.y : fi == 1 ? nb0.w : nb1.y;
+    const float *np = a.h32 + hidx(n1, 0, Nc8, lf);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) cp_async16_cg(E + (fi * 4 + m) * Nc8, np + (F >> (3 * m) & 7) * Nc8);
+    // the second extrapolation point only matters when its coefficient does (wallExtOrder 1
+    // makes it 0)
+    if (e2 == 0.f || code == -1) continue;
     const int cc = -code - 2;
     const float *plane = (cc & 1) ? a.ghostE32[gbuf] : a.ghostW32[gbuf];
-    return plane + ((size_t)(cc >> 1) * 4 + plane_slot(oo)) * Nc8 + lf;
-  };
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int oo = F >> (3 * m) & 7;
+      cp_async16_cg(E + (12 + fi * 4 + m) * Nc8,
+                    code >= 0 ? a.h32 + hidx(code, oo, Nc8, lf)
+                              : plane + ((size_t)(cc >> 1) * 4 + plane_slot(oo)) * Nc8 + lf);
+    }
+  }
+  cp_async_wait_all();
+  float *hn = a.h32 + hidx(r0.x, 0, Nc8, lf), *wn = a.fw32 + hidx(r0.y, 0, Nc8, lf);
   double rho0 = 0.0, rho1 = 0.0, rho2 = 0.0;
   for (int fi = 0; fi < nface; ++fi) {
-    const int dir = P.dir[fi], st = P.store[fi], keep = P.keep[fi];
-    // the face's (neighbour, far point) pair from the record's second half (the same
-    // 128-byte line as its first, so an L1 hit after the loads above)
-    const int2 nbp = __ldg(reinterpret_cast<const int2 *>(rp + 2) + fi);
-    const int n1 = nbp.x, code = nbp.y;
-    double racc = 0.0;
-    if (lv) {
-      float nv[4][VPL], fv[4][VPL];
+    const uint32_t F = P.face[fi];
+    const int dir = F >> 12 & 7, code = fi == 0 ? nb0.y : fi == 1 ? nb0.w : nb1.y;
+    const bool far = e2 != 0.f && code != -1;
+    float *out = (F >> 15 & 3) == ST_F ? hn : wn;
+    float ext[4][4];
 #pragma unroll
-      for (int mm = 0; mm < 4; ++mm) {
-        const int oo = c32_incoming[dir][mm] - 1;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) fv[mm][v] = 0.f;
-        ld32<VPL>(a.h32 + hidx(n1, oo, Nc8, lf), nv[mm]);
-        const float *fp = far_ptr(code, oo);
-        if (fp) ld32<VPL>(fp, fv[mm]);
-      }
-      float ext[4][VPL];
-#pragma unroll
-      for (int mm = 0; mm < 4; ++mm) {
-        const int oo = c32_incoming[dir][mm] - 1;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) ext[mm][v] = e1 * nv[mm][v] + e2 * fv[mm][v];
-        st32<VPL>(E + (size_t)(fi * 4 + mm) * Nc8 + lf, ext[mm]);
-        if (keep >> mm & 1) {
-          if (st == ST_F) st32<VPL>(a.h32 + hidx(node, oo, Nc8, lf), ext[mm]);
-          else st32<VPL>(a.fw32 + hidx(corner, oo, Nc8, lf), ext[mm]);
-        }
-      }
-      // the four octants of a velocity summed in FP32 (one conversion per velocity rather
-      // than four; FP64 ops and conversions are the kernel's short-scoreboard stalls), the
-      // velocities and lanes in FP64
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int l = lf + v;
-        const double ca = dir < 2 ? __ldg(a.cx + l) : dir < 4 ? __ldg(a.cy + l) : __ldg(a.cz + l);
-        racc += ca * (double)__fadd_rn(__fadd_rn(__fadd_rn(ext[0][v], ext[1][v]), ext[2][v]), ext[3][v]);
-      }
+    for (int m = 0; m < 4; ++m) {
+      float *e = E + (fi * 4 + m) * Nc8;
+      const float4 nv = *reinterpret_cast<const float4 *>(e);
+      float4 fv = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (far) fv = *reinterpret_cast<const float4 *>(e + 12 * Nc8);
+      ext[m][0] = e1 * nv.x + e2 * fv.x;
+      ext[m][1] = e1 * nv.y + e2 * fv.y;
+      ext[m][2] = e1 * nv.z + e2 * fv.z;
+      ext[m][3] = e1 * nv.w + e2 * fv.w;
+      st32<4>(e, ext[m]);
+      if (F >> (17 + m) & 1) st32<4>(out + (F >> (3 * m) & 7) * Nc8, ext[m]);
     }
-    // segment sum in FP64 (the FP32 path does not keep the reference's summation order)
-    for (int off = LANES / 2; off > 0; off >>= 1) racc += __shfl_xor_sync(seg, racc, off, LANES);
+    // the four octants of a velocity summed in FP32 (one conversion per velocity rather than
+    // four), the velocities and lanes in FP64
+    const double2 *cp = reinterpret_cast<const double2 *>((dir < 2 ? a.cx : dir < 4 ? a.cy : a.cz) + lf);
+    const double2 c01 = __ldg(cp), c23 = __ldg(cp + 1);
+    const double ca[4] = {c01.x, c01.y, c23.x, c23.y};
+    double tv[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) tv[v] = (double)__fadd_rn(__fadd_rn(__fadd_rn(ext[0][v], ext[1][v]), ext[2][v]), ext[3][v]);
+    double racc;
+    if (LANES == 2) {
+      // velocities l and l + 4 first, then l and l + 2, then the two left
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        tv[v] = __dmul_rn(ca[v], tv[v]);
+        tv[v] += __shfl_xor_sync(seg, tv[v], 1, LANES);
+      }
+      racc = (tv[0] + tv[2]) + (tv[1] + tv[3]);
+    } else {
+      racc = 0.0;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) racc = __fma_rn(ca[v], tv[v], racc);
+#pragma unroll
+      for (int off = LANES / 2; off > 0; off >>= 1) racc += __shfl_xor_sync(seg, racc, off, LANES);
+    }
     if (fi == 0) rho0 = racc; else if (fi == 1) rho1 = racc; else rho2 = racc;
   }
-  if (!lv) return;
   // re-emission in FP32: accom * rho_face rounded once per face, then w * that + (1 - accom)
   // * the extrapolated value, with the weights rounded to FP32 (vtab32 column 3)
-  const float af[3] = {(float)(a.accom * (rho0 / a.DiffFlux)), (float)(a.accom * (rho1 / a.DiffFlux)),
-                       (float)(a.accom * (rho2 / a.DiffFlux))};
+  const float af[3] = {(float)(a.accom * (rho0 / a.DiffFlux)), nface > 1 ? (float)(a.accom * (rho1 / a.DiffFlux)) : 0.f,
+                       nface > 2 ? (float)(a.accom * (rho2 / a.DiffFlux)) : 0.f};
   const float one_m = (float)(1.0 - a.accom);
-  float wl[VPL];
+  float wl[4];
 #pragma unroll
-  for (int v = 0; v < VPL; ++v) wl[v] = __ldg(a.vtab32 + (size_t)(lf + v) * kVtab + 3);
-  for (int k = 0; k < P.nwr; ++k) {
-    const float *sp = E + (size_t)P.src[k] * Nc8 + lf;
-    const float rf = P.face[k] == 0 ? af[0] : P.face[k] == 1 ? af[1] : af[2];
-    float val[VPL];
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) val[v] = __fmaf_rn(rf, wl[v], __fmul_rn(one_m, sp[v]));
-    if (P.dst_store[k] == ST_F) st32<VPL>(a.h32 + hidx(node, P.dst_o[k], Nc8, lf), val);
-    else st32<VPL>(a.fw32 + hidx(corner, P.dst_o[k], Nc8, lf), val);
+  for (int v = 0; v < 4; ++v) wl[v] = __ldg(a.vtab32 + (size_t)(lf + v) * kVtab + 3);
+  const int nwr = (int)P.nwr;
+  for (int k = 0; k < nwr; ++k) {
+    const uint32_t W = P.wr[k];
+    const float4 sp = *reinterpret_cast<const float4 *>(E + (W & 15) * Nc8);
+    const int f = W >> 8 & 3;
+    const float rf = f == 0 ? af[0] : f == 1 ? af[1] : af[2];
+    const float val[4] = {__fmaf_rn(rf, wl[0], __fmul_rn(one_m, sp.x)), __fmaf_rn(rf, wl[1], __fmul_rn(one_m, sp.y)),
+                          __fmaf_rn(rf, wl[2], __fmul_rn(one_m, sp.z)), __fmaf_rn(rf, wl[3], __fmul_rn(one_m, sp.w))};
+    st32<4>((W >> 10 & 1 ? hn : wn) + (W >> 4 & 7) * Nc8, val);
   }
 }
 
@@ -502,23 +526,24 @@ void launch_commit32(const DevState &s, cudaStream_t st) {
 void launch_capture32(const DevState &s, int buf, cudaStream_t st) {
   k_capture32<<<nblocks((size_t)s.Ny * s.Nz * 4 * s.Nc8, 256), 256, 0, st>>>(s, buf);
 }
+namespace {
+template <int LANES>
+void launch_walls32_rows(const DevState &s, int begin, int end, int gbuf, cudaStream_t st) {
+  const int walls = 64 / LANES, far_rows = s.wall_far ? 12 : 0;
+  once_per_device(reinterpret_cast<const void *>(k_walls32_rows<LANES>), [](int) {
+    cudaFuncSetAttribute(k_walls32_rows<LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(float) * wall32_floats(4 * LANES, 12) * (64 / LANES));
+  });
+  const size_t smem = sizeof(float) * (size_t)wall32_floats(s.Nc8, far_rows) * walls;
+  k_walls32_rows<LANES><<<(end - begin + walls - 1) / walls, 64, smem, st>>>(s, begin, end, gbuf, far_rows);
+}
+}  // namespace
 void launch_walls32(const DevState &s, int begin, int end, int gbuf, cudaStream_t st) {
   if (end <= begin) return;
   const size_t walls = (size_t)(end - begin);
-  if (g32_plan_ok && (s.Nc8 == 64 || s.Nc8 <= 32)) {
-    once_per_device(reinterpret_cast<const void *>(k_walls32_onchip<4, 16>), [](int) {
-      cudaFuncSetAttribute(k_walls32_onchip<4, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 12 * 64 * 4);
-    });
-    const size_t smem_per_wall = (size_t)12 * s.Nc8 * sizeof(float);
-    if (s.Nc8 == 64)
-      k_walls32_onchip<4, 16><<<nblocks(walls * 16, 256), 256, 16 * smem_per_wall, st>>>(s, begin, end, gbuf);
-    else if (s.Nc8 <= 8)
-      k_walls32_onchip<1, 8><<<nblocks(walls * 8, 256), 256, 32 * smem_per_wall, st>>>(s, begin, end, gbuf);
-    else k_walls32_onchip<1, 32><<<nblocks(walls * 32, 256), 256, 8 * smem_per_wall, st>>>(s, begin, end, gbuf);
-    return;
-  }
+  if (g32_plan_ok && s.Nc8 == 64) return launch_walls32_rows<16>(s, begin, end, gbuf, st);
+  if (g32_plan_ok && s.Nc8 == 8) return launch_walls32_rows<2>(s, begin, end, gbuf, st);
   if (s.Nc8 % 64 == 0) k_walls32<4, 16><<<nblocks(walls * 16, 256), 256, 0, st>>>(s, begin, end, gbuf);
-  else if (s.Nc8 == 8) k_walls32<1, 8><<<nblocks(walls * 8, 256), 256, 0, st>>>(s, begin, end, gbuf);
   else k_walls32<1, 32><<<nblocks(walls * 32, 256), 256, 0, st>>>(s, begin, end, gbuf);
 }
 void launch_inlet_outlet32(const DevState &s, int buf, cudaStream_t st) {

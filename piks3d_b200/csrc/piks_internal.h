@@ -66,12 +66,13 @@ extern const int kIncoming[6][4];  // 1-based octants arriving from each fluid s
 // write reads it from there; a face value is stored only where no write later replaces
 // it (the slot's final content is then the face value).
 struct WPlan {
-  int nface;
-  int dir[3], store[3];
-  int keep[3];        // per face: bit m set when v(face, m) is the final content of its slot
-  int nwr;
-  int dst_store[12], dst_o[12], face[12];  // 0-based destination octant
-  int src[12];        // producing face * 4 + m
+  uint32_t nface, nwr;
+  // per face: octants of its four values (0-based, 3 bits each) | dir << 12 | store << 15 |
+  // bit 17 + m set when v(face, m) is the final content of its slot
+  uint32_t face[3];
+  // per write: producing face * 4 + m | destination octant << 4 | density face << 8 |
+  // (destination is a slot of the wall node) << 10
+  uint32_t wr[12];
 };
 // Resolves `p`; false if some write reads a value that is not a face extrapolation, reads
 // a slot that an earlier write replaced, or two writes share a destination.
