@@ -383,102 +383,66 @@ __global__ void k_symmetry32(const DevState a) {
   if (f & 8) { hp[4 * S] = hp[0 * S]; hp[5 * S] = hp[1 * S]; hp[6 * S] = hp[2 * S]; hp[7 * S] = hp[3 * S]; }
 }
 
-// Moments in FP64 from FP32 values: LANES lanes per node (32 / LANES nodes per warp), VPL
-// velocities per lane, partial sums combined with a segment reduction (the FP32 path does
-// not follow the reference's order). A whole warp per node measured fastest for 512
-// velocities (half a warp with 16-byte rows: 0.40 vs 0.37 ms on a 128^3 pack).
-template <int VPL, int LANES>
+// Moments in FP64 from FP32 values: LANES lanes over K nodes, two velocities per lane and pass
+// (the FP32 path does not follow the reference's order), all rows of a pass in flight together.
+// The lanes' 4 * K sums are added by halves: at each step a lane keeps one half of its sums and
+// hands the other to its partner, so 9 exchanges serve two nodes of 32 lanes where a tree per sum
+// takes 40; the pairs added are the tree's. What bounds
+// it: the bytes of f (128^3 pack, 512 velocities: 0.342 ms with trees, 0.275 now, 0.263 at the copy
+// rate). Octants of 8 velocities take 4 lanes a node (96^3 pack: 0.164 -> 0.026 ms; a whole warp had
+// 28 idle lanes).
+template <int LANES, int K, int NC8>
 __global__ void __launch_bounds__(256) k_moments32(const DevState a) {
-  const int node = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / LANES);
-  if (node >= a.NF) return;  // whole segment
+  const int node0 = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / LANES) * K;
+  if (node0 >= a.NF) return;  // whole segment
   const int lane = threadIdx.x % LANES;
-  const unsigned seg = LANES == 32 ? 0xffffffffu : (((1u << LANES) - 1u) << (threadIdx.x & 31 & ~(LANES - 1)));
-  const int Nc8 = a.Nc8;
-  const float *hp = a.h32 + (size_t)node * 8 * Nc8;
-  double r = 0.0, ux = 0.0, uy = 0.0, uz = 0.0;
-  for (int l0 = lane * VPL; l0 < Nc8; l0 += LANES * VPL) {
-    float f[8][VPL];
+  const unsigned seg = LANES == 32 ? 0xffffffffu : (((1u << (LANES & 31)) - 1u) << (threadIdx.x & 31 & ~(LANES - 1)));
+  const int Nc8 = NC8 ? NC8 : a.Nc8;
+  double acc[4 * K];
 #pragma unroll
-    for (int o = 0; o < 8; ++o) {
-      if constexpr (VPL == 2) {
-        const float2 t = __ldcs(reinterpret_cast<const float2 *>(hp + (size_t)o * Nc8 + l0));
-        f[o][0] = t.x; f[o][VPL - 1] = t.y;
-      } else {
-        f[o][0] = __ldcs(hp + (size_t)o * Nc8 + l0);
+  for (int i = 0; i < 4 * K; ++i) acc[i] = 0.0;
+  for (int l0 = lane * 2; l0 < Nc8; l0 += LANES * 2) {
+    float2 f[K][8];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float *hp = a.h32 + (size_t)min(node0 + k, a.NF - 1) * 8 * Nc8 + l0;
+#pragma unroll
+      for (int o = 0; o < 8; ++o) f[k][o] = __ldcs(reinterpret_cast<const float2 *>(hp + (size_t)o * Nc8));
+    }
+    const double2 cx = __ldg(reinterpret_cast<const double2 *>(a.cx + l0)),
+                  cy = __ldg(reinterpret_cast<const double2 *>(a.cy + l0)),
+                  cz = __ldg(reinterpret_cast<const double2 *>(a.cz + l0));
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const double f1 = v ? f[k][0].y : f[k][0].x, f2 = v ? f[k][1].y : f[k][1].x, f3 = v ? f[k][2].y : f[k][2].x,
+                     f4 = v ? f[k][3].y : f[k][3].x, f5 = v ? f[k][4].y : f[k][4].x, f6 = v ? f[k][5].y : f[k][5].x,
+                     f7 = v ? f[k][6].y : f[k][6].x, f8 = v ? f[k][7].y : f[k][7].x;
+        acc[4 * k] += ((f1 + f2) + (f3 + f4)) + ((f5 + f6) + (f7 + f8));
+        acc[4 * k + 1] += (v ? cx.y : cx.x) * (((f1 - f2) + (f4 - f3)) + ((f5 - f6) + (f8 - f7)));
+        acc[4 * k + 2] += (v ? cy.y : cy.x) * (((f1 + f2) - (f3 + f4)) + ((f5 + f6) - (f7 + f8)));
+        acc[4 * k + 3] += (v ? cz.y : cz.x) * (((f1 + f2) + (f3 + f4)) - ((f5 + f6) + (f7 + f8)));
       }
-    }
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      const int l = l0 + v;
-      const double f1 = f[0][v], f2 = f[1][v], f3 = f[2][v], f4 = f[3][v], f5 = f[4][v], f6 = f[5][v],
-                   f7 = f[6][v], f8 = f[7][v];
-      r += ((f1 + f2) + (f3 + f4)) + ((f5 + f6) + (f7 + f8));
-      ux += __ldg(a.cx + l) * (((f1 - f2) + (f4 - f3)) + ((f5 - f6) + (f8 - f7)));
-      uy += __ldg(a.cy + l) * (((f1 + f2) - (f3 + f4)) + ((f5 + f6) - (f7 + f8)));
-      uz += __ldg(a.cz + l) * (((f1 + f2) + (f3 + f4)) - ((f5 + f6) + (f7 + f8)));
-    }
   }
+  int n = 4 * K, which = 0;
+#pragma unroll
   for (int off = LANES / 2; off > 0; off >>= 1) {
-    r += __shfl_down_sync(seg, r, off, LANES);
-    ux += __shfl_down_sync(seg, ux, off, LANES);
-    uy += __shfl_down_sync(seg, uy, off, LANES);
-    uz += __shfl_down_sync(seg, uz, off, LANES);
-  }
-  if (lane == 0) {
-    double2 *mp = reinterpret_cast<double2 *>(a.mom) + 2 * (size_t)node;
-    mp[0] = make_double2(r, ux);
-    mp[1] = make_double2(uy, uz);
-  }
-}
-
-// The same sums for 64 velocities per octant, a warp over two nodes at a time: the sixteen
-// row loads of both nodes are in flight together (each node's sums as in k_moments32).
-__global__ void __launch_bounds__(256) k_moments32_pair(const DevState a) {
-  const int node0 = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2;
-  if (node0 >= a.NF) return;  // whole warp
-  const int lane = threadIdx.x & 31;
-  const int l0 = lane * 2;
-  const bool two = node0 + 1 < a.NF;
-  float f[2][8][2];
+    if (n > 1) {
+      n /= 2;
+      const bool up = lane & off;
+      if (up) which += n;
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const float *hp = a.h32 + (size_t)(two ? node0 + k : node0) * 8 * 64;
-#pragma unroll
-    for (int o = 0; o < 8; ++o) {
-      const float2 t = __ldcs(reinterpret_cast<const float2 *>(hp + (size_t)o * 64 + l0));
-      f[k][o][0] = t.x; f[k][o][1] = t.y;
+      for (int i = 0; i < n; ++i) {
+        const double mine = up ? acc[i + n] : acc[i], theirs = up ? acc[i] : acc[i + n];
+        acc[i] = mine + __shfl_xor_sync(seg, theirs, off, LANES);
+      }
+    } else {
+      acc[0] += __shfl_xor_sync(seg, acc[0], off, LANES);
     }
   }
-  const double cx0 = __ldg(a.cx + l0), cx1 = __ldg(a.cx + l0 + 1), cy0 = __ldg(a.cy + l0), cy1 = __ldg(a.cy + l0 + 1),
-               cz0 = __ldg(a.cz + l0), cz1 = __ldg(a.cz + l0 + 1);
-  double acc[2][4];
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    double r = 0.0, ux = 0.0, uy = 0.0, uz = 0.0;
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-      const double f1 = f[k][0][v], f2 = f[k][1][v], f3 = f[k][2][v], f4 = f[k][3][v], f5 = f[k][4][v],
-                   f6 = f[k][5][v], f7 = f[k][6][v], f8 = f[k][7][v];
-      r += ((f1 + f2) + (f3 + f4)) + ((f5 + f6) + (f7 + f8));
-      ux += (v ? cx1 : cx0) * (((f1 - f2) + (f4 - f3)) + ((f5 - f6) + (f8 - f7)));
-      uy += (v ? cy1 : cy0) * (((f1 + f2) - (f3 + f4)) + ((f5 + f6) - (f7 + f8)));
-      uz += (v ? cz1 : cz0) * (((f1 + f2) + (f3 + f4)) - ((f5 + f6) + (f7 + f8)));
-    }
-    acc[k][0] = r; acc[k][1] = ux; acc[k][2] = uy; acc[k][3] = uz;
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[k][q] += __shfl_down_sync(0xffffffffu, acc[k][q], off);
-  if (lane == 0) {
-    for (int k = 0; k < (two ? 2 : 1); ++k) {
-      double2 *mp = reinterpret_cast<double2 *>(a.mom) + 2 * (size_t)(node0 + k);
-      mp[0] = make_double2(acc[k][0], acc[k][1]);
-      mp[1] = make_double2(acc[k][2], acc[k][3]);
-    }
-  }
+  constexpr int kSame = LANES / (4 * K);  // lanes left with the same sum
+  if (lane % kSame == 0 && node0 + which / 4 < a.NF) a.mom[(size_t)node0 * 4 + which] = acc[0];
 }
 
 __global__ void k_widen(const float *src, double *dst, size_t n) {
@@ -554,9 +518,9 @@ void launch_symmetry32(const DevState &s, cudaStream_t st) {
 }
 void launch_moments32(const DevState &s, cudaStream_t st) {
   if (!s.NF) return;
-  if (s.Nc8 == 64) k_moments32_pair<<<nblocks((size_t)(s.NF + 1) / 2 * 32, 256), 256, 0, st>>>(s);
-  else if (s.Nc8 % 2 == 0) k_moments32<2, 32><<<nblocks((size_t)s.NF * 32, 256), 256, 0, st>>>(s);
-  else k_moments32<1, 32><<<nblocks((size_t)s.NF * 32, 256), 256, 0, st>>>(s);
+  if (s.Nc8 == 8) k_moments32<4, 1, 8><<<nblocks((size_t)s.NF * 4, 256), 256, 0, st>>>(s);
+  else if (s.Nc8 == 64) k_moments32<32, 2, 64><<<nblocks((size_t)(s.NF + 1) / 2 * 32, 256), 256, 0, st>>>(s);
+  else k_moments32<32, 2, 0><<<nblocks((size_t)(s.NF + 1) / 2 * 32, 256), 256, 0, st>>>(s);
 }
 template <typename T>
 __global__ void __launch_bounds__(256) k_gram(const char *base, size_t stride, int n, size_t count, double *partial) {
