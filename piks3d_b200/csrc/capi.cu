@@ -98,13 +98,56 @@ void release(piks_ctx *c, void *p) {
     }
 }
 
+// Pinned slices for fetch_macro, kept between calls while some device context lives: a call
+// borrows a stage (the first of a process takes 2 to 3 ms to allocate), at most two wait here,
+// of at most 16 slices of 256 KiB each.
+struct MacroStage { double *p; int slices; };
+struct StagePool {
+  std::mutex lock;
+  std::vector<MacroStage> idle;
+  int contexts = 0;
+  MacroStage take(int slices, size_t slice) {
+    {
+      std::lock_guard<std::mutex> hold(lock);
+      for (size_t i = 0; i < idle.size(); ++i)
+        if (idle[i].slices >= slices) {
+          const MacroStage s = idle[i];
+          idle.erase(idle.begin() + (long)i);
+          return s;
+        }
+    }
+    MacroStage s{nullptr, slices};
+    if (cudaMallocHost(&s.p, slice * slices * sizeof(double)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      s.p = nullptr;
+    }
+    return s;
+  }
+  void give(MacroStage s) {
+    if (!s.p) return;
+    std::lock_guard<std::mutex> hold(lock);
+    if (contexts > 0 && idle.size() < 2) { idle.push_back(s); return; }
+    for (auto &i : idle)
+      if (i.slices < s.slices) std::swap(i, s);
+    cudaFreeHost(s.p);
+  }
+  void context(int change) {
+    std::lock_guard<std::mutex> hold(lock);
+    contexts += change;
+    if (contexts > 0) return;
+    for (auto &i : idle) cudaFreeHost(i.p);
+    idle.clear();
+  }
+};
+StagePool g_macro_stages;
+
 // The moments into the box's fields (0 at non-fluid voxels): blocks of kMacroNodes fluid nodes,
 // which are numbered in raster order, so that a block owns the voxels from its first node to the
 // next block's. Host threads take blocks: a block's moments come over into the thread's pinned
 // slice, then each field's part is zeroed and filled while it is in the cache. What bounds it is
 // the first touch of the caller's pages. One thread, a whole pageable copy and four passes over
 // the box took 1.1 / 2.2 / 50 / 250 ms for boxes of 32^3 / 48^3 / 128^3 / 256^3 voxels; this takes
-// 0.25 / 0.45 / 3 / 18 ms on 16 cores (the first call, which allocates the slices, 0.5 / 0.7 / 4 / 19).
+// 0.25 / 0.45 / 3 / 18 ms on 16 cores (a process's first call allocates the slices: 2 to 3 ms more).
 constexpr int64_t kMacroNodes = 8192;
 cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
   const Geometry &g = c->geo;
@@ -112,20 +155,12 @@ cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
   const unsigned hw = std::thread::hardware_concurrency();
   const int nw = (int)std::min<int64_t>(std::max(1u, std::min(hw ? hw : 1u, 16u)), nblock);
   const size_t slice = (size_t)kMacroNodes * 4;
-  std::lock_guard<std::mutex> hold(c->macro_lock);
+  const MacroStage pinned = g_macro_stages.take(nw, slice);
   std::vector<double> pageable;
-  if (c->macro_slices < nw) {
-    if (c->macro_stage) cudaFreeHost(c->macro_stage);
-    c->macro_stage = nullptr;
-    c->macro_slices = 0;
-    if (cudaMallocHost(&c->macro_stage, slice * nw * sizeof(double)) == cudaSuccess) c->macro_slices = nw;
-    else {
-      (void)cudaGetLastError();
-      c->macro_stage = nullptr;
-      try { pageable.resize(slice * nw); } catch (const std::bad_alloc &) { return cudaErrorMemoryAllocation; }
-    }
+  if (!pinned.p) {
+    try { pageable.resize(slice * nw); } catch (const std::bad_alloc &) { return cudaErrorMemoryAllocation; }
   }
-  double *stage = c->macro_stage ? c->macro_stage : pageable.data();
+  double *stage = pinned.p ? pinned.p : pageable.data();
   const int64_t box = (int64_t)g.Nx * g.Ny * g.Nz;
   auto voxel = [&](int64_t n) -> int64_t {
     const uint32_t gi = (uint32_t)g.node_g[(size_t)n], gx = (uint32_t)g.GX, gy = (uint32_t)g.GY;
@@ -167,6 +202,8 @@ cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
   }
   work(0);
   for (auto &t : th) t.join();
+  if (status != (int)cudaSuccess) cudaStreamSynchronize(c->stream);  // no copy is left under way
+  g_macro_stages.give(pinned);
   return (cudaError_t)status.load();
 }
 
@@ -669,6 +706,7 @@ piks_status piks_create(const piks_params *p, int32_t device, piks_ctx **out) {
       uploaded |= 1ull << (device & 63);
     }
   }
+  g_macro_stages.context(1);
   *out = c;
   return PIKS_OK;
 }
@@ -1763,7 +1801,7 @@ piks_status piks_destroy(piks_ctx *c) {
   cudaStreamSynchronize(c->stream);
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   free_device(c);
-  if (c->macro_stage) cudaFreeHost(c->macro_stage);
+  g_macro_stages.context(-1);
   if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;

@@ -3,7 +3,6 @@
 #include <cuda_runtime.h>
 
 #include <future>
-#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -55,10 +54,6 @@ struct piks_ctx {
   size_t snap_bytes = 0;
   int snap_prec = -1, snap_version = -1;
   int snap_steps[8] = {-1, -1, -1, -1, -1, -1, -1, -1};  // iteration of each slot's copy
-  // pinned slices the fields come over through (fetch_macro), at most 16 of 256 KiB
-  double *macro_stage = nullptr;
-  int macro_slices = 0;
-  std::mutex macro_lock;
   double mass = 1.0, error = 1.0, permeability = 0.0;
   bool timing = false;
   double kt_ms[piks::KT_N] = {0};
