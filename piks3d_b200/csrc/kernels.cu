@@ -10,6 +10,7 @@
 #include <set>
 #include <tuple>
 
+#include "boundary.cuh"
 #include "kernels.h"
 #include "piks_internal.h"
 
@@ -182,24 +183,6 @@ __global__ void k_commit16(const int32_t *commit, const int32_t *bcorner, int NF
   const int4 v = src < 8 ? h[((size_t)node * 8 + src) * pieces + pc]
                          : fw[((size_t)bcorner[node - NF] * 8 + o) * pieces + pc];
   h[((size_t)node * 8 + o) * pieces + pc] = v;
-}
-
-// Periodic x halo (solver.F90:535-560, one rank): the planes x = Nx (octants with cx > 0)
-// and x = 1 (cx < 0) as they stand after the sweep become the ghost planes x = 0 and
-// x = Nx+1 that the boundary conditions of the NEXT iteration read.
-__global__ void k_capture(const DevState a, int buf) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t rows = (size_t)a.Ny * a.Nz;
-  const size_t total = rows * 4 * a.Nc8;
-  if (idx >= total) return;
-  const int l = (int)(idx % a.Nc8);
-  const int q = (int)((idx / a.Nc8) % 4);
-  const size_t r = idx / ((size_t)a.Nc8 * 4);
-  const int oW = (q == 0) ? 0 : (q == 1) ? 3 : (q == 2) ? 4 : 7;   // cx > 0
-  const int oE = (q == 0) ? 1 : (q == 1) ? 2 : (q == 2) ? 5 : 6;   // cx < 0
-  const int nW = a.plane_xN[r], nE = a.plane_x1[r];
-  a.ghostW[buf][idx] = nW >= 0 ? a.h[hidx(nW, oW, a.Nc8, l)] : 0.0;
-  a.ghostE[buf][idx] = nE >= 0 ? a.h[hidx(nE, oE, a.Nc8, l)] : 0.0;
 }
 
 // Diffuse wall (solver.F90:761-1826): one warp per wall, lanes over velocities (VPL per
@@ -472,44 +455,6 @@ k_walls_rows(const DevState a, int begin, int end, int gbuf, int far_rows) {
     for (int v = 0; v < 2; ++v) val[v] = dadd(dmul(aw[v], r), dmul(one_m, src[v]));
     st_vpl<2>((W >> 10 & 1 ? hn : wn) + (W >> 4 & 7) * Nc8, val);
   }
-}
-
-// Inlet x = 1 and outlet x = Nx with the pressure jump (solver.F90:1832-1862), reading the
-// ghost planes captured in the previous iteration.
-__global__ void k_inlet_outlet(const DevState a, int gbuf) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t total = (size_t)a.Ny * a.Nz * 4 * a.Nc8;
-  if (idx >= total) return;
-  const int l = (int)(idx % a.Nc8);
-  const int q = (int)((idx / a.Nc8) % 4);
-  const size_t r = idx / ((size_t)a.Nc8 * 4);
-  const double wdp = dmul(a.w[l], a.pressDrop);
-  const int n1 = a.plane_x1[r], nN = a.plane_xN[r];
-  if (n1 >= 0) {
-    const int o = (q == 0) ? 0 : (q == 1) ? 3 : (q == 2) ? 4 : 7;
-    a.h[hidx(n1, o, a.Nc8, l)] = dadd(a.ghostW[gbuf][idx], wdp);
-  }
-  if (nN >= 0) {
-    const int o = (q == 0) ? 1 : (q == 1) ? 2 : (q == 2) ? 5 : 6;
-    a.h[hidx(nN, o, a.Nc8, l)] = dsub(a.ghostE[gbuf][idx], wdp);
-  }
-}
-
-// Specular symmetry planes y = 1, y = Ny, z = 1, z = Nz in the reference's order
-// (solver.F90:1867-1918).
-__global__ void k_symmetry(const DevState a) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t total = (size_t)a.nsym * a.Nc8;
-  if (idx >= total) return;
-  const int s = (int)(idx / a.Nc8), l = (int)(idx % a.Nc8);
-  const int n = a.sym_node[s];
-  const uint8_t f = a.sym_flag[s];
-  double *hp = a.h + (size_t)n * 8 * a.Nc8 + l;
-  const size_t S = a.Nc8;
-  if (f & 1) { hp[1 * S] = hp[2 * S]; hp[0 * S] = hp[3 * S]; hp[5 * S] = hp[6 * S]; hp[4 * S] = hp[7 * S]; }
-  if (f & 2) { hp[2 * S] = hp[1 * S]; hp[3 * S] = hp[0 * S]; hp[6 * S] = hp[5 * S]; hp[7 * S] = hp[4 * S]; }
-  if (f & 4) { hp[0 * S] = hp[4 * S]; hp[1 * S] = hp[5 * S]; hp[2 * S] = hp[6 * S]; hp[3 * S] = hp[7 * S]; }
-  if (f & 8) { hp[4 * S] = hp[0 * S]; hp[5 * S] = hp[1 * S]; hp[6 * S] = hp[2 * S]; hp[7 * S] = hp[3 * S]; }
 }
 
 // Moments Rho, Ux, Uy, Uz (solver.F90:1923-1938). A warp owns 32 fluid nodes; lane n
@@ -944,8 +889,7 @@ void launch_commit(const DevState &s, cudaStream_t st) {
 }
 
 void launch_capture(const DevState &s, int buf, cudaStream_t st) {
-  const size_t n = (size_t)s.Ny * s.Nz * 4 * s.Nc8;
-  k_capture<<<blocks_for(n, 256), 256, 0, st>>>(s, buf);
+  boundary::launch_capture<double>(s.h, s.ghostW[buf], s.ghostE[buf], s, st);
 }
 
 // Halo rows (solver.F90:535-560 for the planes of a slab boundary): element idx of a
@@ -987,15 +931,10 @@ void launch_halo(const DevState &s, bool fp32, int cap, cudaStream_t st) {
 }
 
 void launch_inlet_outlet(const DevState &s, int buf, cudaStream_t st) {
-  const size_t n = (size_t)s.Ny * s.Nz * 4 * s.Nc8;
-  k_inlet_outlet<<<blocks_for(n, 256), 256, 0, st>>>(s, buf);
+  boundary::launch_inlet_outlet<double>(s.h, s.ghostW[buf], s.ghostE[buf], s, st);
 }
 
-void launch_symmetry(const DevState &s, cudaStream_t st) {
-  if (s.nsym == 0) return;
-  const size_t n = (size_t)s.nsym * s.Nc8;
-  k_symmetry<<<blocks_for(n, 256), 256, 0, st>>>(s);
-}
+void launch_symmetry(const DevState &s, cudaStream_t st) { boundary::launch_symmetry<double>(s.h, s, st); }
 
 void launch_moments(const DevState &s, cudaStream_t st) {
   if (s.NF == 0) return;

@@ -6,6 +6,7 @@
 // arithmetic type differs, so the FP32 iterate approximates the FP64 one.
 #include <cuda_runtime.h>
 
+#include "boundary.cuh"
 #include "kernels.h"
 #include "piks_internal.h"
 
@@ -112,19 +113,6 @@ __global__ void k_commit32(const DevState a) {
   const int node = a.commit[3 * e], o = a.commit[3 * e + 1], src = a.commit[3 * e + 2];
   a.h32[hidx(node, o, a.Nc8, l)] = src < 8 ? a.h32[hidx(node, src, a.Nc8, l)]
                                            : a.fw32[hidx(a.bcorner[node - a.NF], o, a.Nc8, l)];
-}
-
-__global__ void k_capture32(const DevState a, int buf) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)a.Ny * a.Nz * 4 * a.Nc8) return;
-  const int l = (int)(idx % a.Nc8);
-  const int q = (int)((idx / a.Nc8) % 4);
-  const size_t r = idx / ((size_t)a.Nc8 * 4);
-  const int oW = q == 0 ? 0 : q == 1 ? 3 : q == 2 ? 4 : 7;
-  const int oE = q == 0 ? 1 : q == 1 ? 2 : q == 2 ? 5 : 6;
-  const int nW = a.plane_xN[r], nE = a.plane_x1[r];
-  a.ghostW32[buf][idx] = nW >= 0 ? a.h32[hidx(nW, oW, a.Nc8, l)] : 0.f;
-  a.ghostE32[buf][idx] = nE >= 0 ? a.h32[hidx(nE, oE, a.Nc8, l)] : 0.f;
 }
 
 // Walls: extrapolation and re-emission in FP32, the wall densities summed in FP64 (a warp
@@ -358,31 +346,6 @@ __global__ void __launch_bounds__(64, 18) k_walls32_rows(const DevState a, int b
   }
 }
 
-__global__ void k_inlet_outlet32(const DevState a, int gbuf) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)a.Ny * a.Nz * 4 * a.Nc8) return;
-  const int l = (int)(idx % a.Nc8);
-  const int q = (int)((idx / a.Nc8) % 4);
-  const size_t r = idx / ((size_t)a.Nc8 * 4);
-  const float wdp = (float)(a.w[l] * a.pressDrop);
-  const int n1 = a.plane_x1[r], nN = a.plane_xN[r];
-  if (n1 >= 0) a.h32[hidx(n1, q == 0 ? 0 : q == 1 ? 3 : q == 2 ? 4 : 7, a.Nc8, l)] = a.ghostW32[gbuf][idx] + wdp;
-  if (nN >= 0) a.h32[hidx(nN, q == 0 ? 1 : q == 1 ? 2 : q == 2 ? 5 : 6, a.Nc8, l)] = a.ghostE32[gbuf][idx] - wdp;
-}
-
-__global__ void k_symmetry32(const DevState a) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)a.nsym * a.Nc8) return;
-  const int s = (int)(idx / a.Nc8), l = (int)(idx % a.Nc8);
-  const uint8_t f = a.sym_flag[s];
-  float *hp = a.h32 + (size_t)a.sym_node[s] * 8 * a.Nc8 + l;
-  const size_t S = a.Nc8;
-  if (f & 1) { hp[1 * S] = hp[2 * S]; hp[0 * S] = hp[3 * S]; hp[5 * S] = hp[6 * S]; hp[4 * S] = hp[7 * S]; }
-  if (f & 2) { hp[2 * S] = hp[1 * S]; hp[3 * S] = hp[0 * S]; hp[6 * S] = hp[5 * S]; hp[7 * S] = hp[4 * S]; }
-  if (f & 4) { hp[0 * S] = hp[4 * S]; hp[1 * S] = hp[5 * S]; hp[2 * S] = hp[6 * S]; hp[3 * S] = hp[7 * S]; }
-  if (f & 8) { hp[4 * S] = hp[0 * S]; hp[5 * S] = hp[1 * S]; hp[6 * S] = hp[2 * S]; hp[7 * S] = hp[3 * S]; }
-}
-
 // Moments in FP64 from FP32 values: LANES lanes over K nodes, two velocities per lane and pass
 // (the FP32 path does not follow the reference's order), all rows of a pass in flight together.
 // The lanes' 4 * K sums are added by halves: at each step a lane keeps one half of its sums and
@@ -488,7 +451,7 @@ void launch_commit32(const DevState &s, cudaStream_t st) {
   if (s.ncommit) k_commit32<<<nblocks((size_t)s.ncommit * s.Nc8, 256), 256, 0, st>>>(s);
 }
 void launch_capture32(const DevState &s, int buf, cudaStream_t st) {
-  k_capture32<<<nblocks((size_t)s.Ny * s.Nz * 4 * s.Nc8, 256), 256, 0, st>>>(s, buf);
+  boundary::launch_capture<float>(s.h32, s.ghostW32[buf], s.ghostE32[buf], s, st);
 }
 namespace {
 template <int LANES>
@@ -511,10 +474,10 @@ void launch_walls32(const DevState &s, int begin, int end, int gbuf, cudaStream_
   else k_walls32<1, 32><<<nblocks(walls * 32, 256), 256, 0, st>>>(s, begin, end, gbuf);
 }
 void launch_inlet_outlet32(const DevState &s, int buf, cudaStream_t st) {
-  k_inlet_outlet32<<<nblocks((size_t)s.Ny * s.Nz * 4 * s.Nc8, 256), 256, 0, st>>>(s, buf);
+  boundary::launch_inlet_outlet<float>(s.h32, s.ghostW32[buf], s.ghostE32[buf], s, st);
 }
 void launch_symmetry32(const DevState &s, cudaStream_t st) {
-  if (s.nsym) k_symmetry32<<<nblocks((size_t)s.nsym * s.Nc8, 256), 256, 0, st>>>(s);
+  boundary::launch_symmetry<float>(s.h32, s, st);
 }
 void launch_moments32(const DevState &s, cudaStream_t st) {
   if (!s.NF) return;
