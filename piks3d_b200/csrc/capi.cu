@@ -454,7 +454,7 @@ bool build_tiles_for(const piks_ctx *c, const int *dims, int form, TileJobs &tj,
 }
 
 // The hyperplane-column schedule of the context's geometry (false: not usable). The columns'
-// cross-section: a batch (one hyperplane of a column) costs some 1100 cycles whatever its size,
+// cross-section: a batch (one hyperplane of a column) costs some 1000 cycles whatever its size,
 // which asks for wide columns, and its rows fill the ring of one SM's shared memory, which has to
 // hold three of the largest batches and wants some to spare for the loads of the next. With rows
 // of 256 bytes (FP64 32, FP32 64 velocities) that is about 700 rows: 10 x 10, or 9 x 9 where most
