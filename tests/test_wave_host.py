@@ -3,6 +3,9 @@ numpy as the kernel runs it - rows copied into a ring of exactly its size as soo
 rule allows (overwriting what it overwrites), tasks reading ring slots only, columns one after
 another in their listed order - and every swept row must equal the per-node task list's result
 bit for bit."""
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -94,3 +97,15 @@ def test_columns_replay_the_per_node_tasks(n, kw):
     got = _replay(s, start.copy())
     assert np.array_equal(got, want)
     s.close()
+
+
+def test_warps_that_may_leave_meet_on_mbarriers_only():
+    """Warps of the column kernel leave one by one once a bounded wait has given up. A counted
+    barrier after that point would wait for the ones that left, without a limit: the kernel's only
+    one is the __syncthreads() before its warps take up their roles."""
+    src = open(os.path.join(os.path.dirname(pk.__file__), "csrc", "sweep_wave.cu")).read()
+    code = re.sub(r"//[^\n]*", "", src)
+    counted = re.findall(r"__syncthreads|\bbar\.(?:sync|red|arrive)|\bbarrier\.(?:cta\.)?(?:sync|red|arrive)|__barrier_sync", code)
+    assert counted == ["__syncthreads"]
+    kernel = code[code.index("k_wave_sweep(const DevState a"):]
+    assert kernel.index("__syncthreads") < kernel.index("setmaxnreg")
