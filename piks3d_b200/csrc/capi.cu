@@ -144,7 +144,10 @@ StagePool g_macro_stages;
 // The moments into the box's fields (0 at non-fluid voxels): blocks of kMacroNodes fluid nodes,
 // which are numbered in raster order, so that a block owns the voxels from its first node to the
 // next block's. Host threads take blocks: a block's moments come over into the thread's pinned
-// slice, then each field's part is zeroed and filled while it is in the cache. What bounds it is
+// slice, then each field's part is zeroed and filled while it is in the cache. The caller's
+// stream may be cudaStreamPerThread, whose handle names another stream in every thread: the
+// calling thread marks the end of the iterations with an event, each host thread waits for it
+// and for its own copies. What bounds it is
 // the first touch of the caller's pages. One thread, a whole pageable copy and four passes over
 // the box took 1.1 / 2.2 / 50 / 250 ms for boxes of 32^3 / 48^3 / 128^3 / 256^3 voxels; this takes
 // 0.25 / 0.45 / 3 / 18 ms on 16 cores (a process's first call allocates the slices: 2 to 3 ms more).
@@ -169,12 +172,16 @@ cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
   };
   std::atomic<int64_t> next{0};
   std::atomic<int> status{(int)cudaSuccess};
+  cudaEvent_t computed = nullptr;
+  cudaError_t marked = cudaEventCreateWithFlags(&computed, cudaEventDisableTiming);
+  if (marked == cudaSuccess) marked = cudaEventRecord(computed, c->stream);
   auto work = [&](int w) {
     cudaSetDevice(c->device);
     double *buf = stage + slice * (size_t)w;
     int32_t at[kMacroNodes];
     cudaEvent_t done;
-    cudaError_t e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+    cudaError_t e = cudaEventSynchronize(computed);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
     if (e != cudaSuccess) { status = (int)e; return; }
     for (int64_t b; (b = next.fetch_add(1)) < nblock && status == (int)cudaSuccess;) {
       const int64_t n0 = b * kMacroNodes, n1 = std::min<int64_t>(g.NF, n0 + kMacroNodes);
@@ -185,7 +192,7 @@ cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
       const int64_t v0 = b == 0 ? 0 : voxel(n0), v1 = n1 == g.NF ? box : voxel(n1);
       for (int64_t n = n0; n < n1; ++n) at[n - n0] = (int32_t)(voxel(n) - v0);
       if (e == cudaSuccess) e = cudaEventSynchronize(done);
-      if (e != cudaSuccess) { status = (int)e; break; }
+      if (e != cudaSuccess) { status = (int)e; cudaStreamSynchronize(c->stream); break; }  // no copy is left under way
       for (int q = 0; q < 4; ++q) {
         if (!dst[q]) continue;
         double *out = dst[q] + v0;
@@ -196,13 +203,17 @@ cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
     cudaEventDestroy(done);
   };
   std::vector<std::thread> th;
-  th.reserve((size_t)nw);
-  for (int w = 1; w < nw; ++w) {
-    try { th.emplace_back(work, w); } catch (const std::system_error &) { break; }  // the others take its blocks
+  if (marked == cudaSuccess) {
+    th.reserve((size_t)nw);
+    for (int w = 1; w < nw; ++w) {
+      try { th.emplace_back(work, w); } catch (const std::system_error &) { break; }  // the others take its blocks
+    }
+    work(0);
+    for (auto &t : th) t.join();
+  } else {
+    status = (int)marked;
   }
-  work(0);
-  for (auto &t : th) t.join();
-  if (status != (int)cudaSuccess) cudaStreamSynchronize(c->stream);  // no copy is left under way
+  if (computed) cudaEventDestroy(computed);
   g_macro_stages.give(pinned);
   return (cudaError_t)status.load();
 }
