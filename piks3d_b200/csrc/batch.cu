@@ -93,6 +93,8 @@ piks_status rebuild(piks_batch *b) {
   drop_graphs(b);
   b->warm = 0;
   const size_t nm = b->members.size();
+  for (const piks_ctx *c : b->members)
+    if (!c->use_wave && !c->use_tiles) return fail(PIKS_ERR_STATE, "a batch member no longer has a column or tile schedule");
   if (nm > b->states_cap) {
     if (b->d_states) cudaFree(b->d_states);
     b->d_states = nullptr;

@@ -506,6 +506,15 @@ bool build_tiles(piks_ctx *c) {
   return c->use_tiles;
 }
 
+// The sweep schedule on the host: columns (`wave`), or the tile jobs of the context's shape and
+// launch schedule, each falling back to the next (columns, tiles, nodes).
+void build_schedule(piks_ctx *c, bool wave) {
+  c->tiles = TileJobs{};
+  c->use_tiles = false;
+  c->use_wave = wave && build_wave(c);
+  if (!c->use_wave) build_tiles(c);
+}
+
 // The velocity chunks and items of the columns for the state's precision.
 void wave_precision(piks_ctx *c) {
   WaveView &w = c->ds.wv;
@@ -619,6 +628,30 @@ piks_status upload_tiles(piks_ctx *c) {
     tv.ncols = (int)tj.col_list.size();
   }
   return PIKS_OK;
+}
+
+// Device copy of the context's schedule. A context whose upload fails has none (piks_iterate
+// refuses it) until the next set-up or change of schedule.
+piks_status upload_schedule(piks_ctx *c) {
+  piks_status st = upload_wave(c);
+  if (!st) st = upload_tiles(c);
+  if (st) c->use_wave = c->use_tiles = false;
+  return st;
+}
+
+// f, fw, the ghost planes and the moments back to setupFlow's zeros.
+piks_status reset_state(piks_ctx *c) {
+  const StateSizes z = state_sizes(c);
+  DevState &s = c->ds;
+  const bool f32 = c->prec == PIKS_PREC_FP32;
+  const size_t e = f32 ? sizeof(float) : sizeof(double);
+  cudaMemsetAsync(f32 ? (void *)s.h32 : (void *)s.h, 0, (z.h + z.fw) * e, c->stream);
+  for (int b = 0; b < 2; ++b) {
+    cudaMemsetAsync(f32 ? (void *)s.ghostW32[b] : (void *)s.ghostW[b], 0, z.plane * e, c->stream);
+    cudaMemsetAsync(f32 ? (void *)s.ghostE32[b] : (void *)s.ghostE[b], 0, z.plane * e, c->stream);
+  }
+  cudaMemsetAsync(s.mom, 0, (size_t)c->geo.NF * 4 * sizeof(double), c->stream);
+  return cuda_check(cudaStreamSynchronize(c->stream), "autotune reset");
 }
 
 }  // namespace
@@ -758,11 +791,8 @@ piks_status piks_setup_physical_grid(piks_ctx *c, const uint8_t *raw, int64_t nb
   c->have_host_geometry = true;
   c->tiles_tuned = false;
   if (!c->tiles_explicit) default_tile_dims(c->prec, c->tile_dims);
-  c->tiles = TileJobs{};
-  c->use_tiles = false;
   c->wave_items[0] = c->wave_items[1] = nullptr;
-  c->use_wave = c->schedule == PIKS_SCHED_WAVE && build_wave(c);
-  if (!c->use_wave) build_tiles(c);
+  build_schedule(c, c->schedule == PIKS_SCHED_WAVE);
   if (c->device < 0) {
     c->setup_seconds[3] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_setup).count();
     return PIKS_OK;
@@ -904,6 +934,8 @@ piks_status piks_iterate(piks_ctx *c, int32_t nsteps) {
   if (c->device < 0) return fail(PIKS_ERR_NOT_FOUND, "host-only context (device -1) cannot iterate");
   if (!c->have_geometry) return fail(PIKS_ERR_STATE, "piks_setup_physical_grid has not been called");
   if (nsteps < 0) return fail(PIKS_ERR_ARG, "nsteps < 0");
+  if (!c->use_wave && !c->use_tiles && !c->ds.tasks && !c->geo.tasks.empty())
+    return fail(PIKS_ERR_STATE, "no sweep schedule on the device (its upload failed): set the image up again");
   if (c->setup.nranks > 1 && nsteps > 1)
     return fail(PIKS_ERR_ARG, "a slab context iterates one step per call (its halos are exchanged between calls)");
   cudaSetDevice(c->device);
@@ -1198,7 +1230,7 @@ static piks_status retile_for_precision(piks_ctx *c) {
   if (!ok) return PIKS_OK;  // keep the current schedule
   c->tiles = std::move(tj);
   c->tile_dims[0] = d[0]; c->tile_dims[1] = d[1]; c->tile_dims[2] = d[2];
-  piks_status st = upload_tiles(c);
+  piks_status st = upload_schedule(c);
   if (!st) st = cuda_check(cudaStreamSynchronize(c->stream), "retile");
   return st;
 }
@@ -1252,7 +1284,7 @@ piks_status piks_set_precision(piks_ctx *c, int32_t precision) {
   if (c->use_tiles && !c->tiles.split && c->tiles.plan_prec != precision) {
     // the schedule stayed: its launch plan becomes the new precision's
     plan_for_precision(c->tiles, precision);
-    if ((st = upload_tiles(c))) return st;
+    if ((st = upload_schedule(c))) return st;
     if ((st = cuda_check(cudaStreamSynchronize(c->stream), "replan"))) return st;
   }
   c->version += 1;
@@ -1287,13 +1319,9 @@ piks_status piks_set_schedule(piks_ctx *c, int32_t schedule) {
     piks_status st = cuda_check(cudaStreamSynchronize(c->stream), "schedule sync");
     if (st) return st;
   }
-  c->tiles = TileJobs{};
-  c->use_tiles = false;
-  c->use_wave = wave && build_wave(c);
-  if (!c->use_wave) build_tiles(c);
+  build_schedule(c, wave);
   if (c->device >= 0 && c->have_geometry) {
-    piks_status st = upload_wave(c);
-    if (!st) st = upload_tiles(c);
+    piks_status st = upload_schedule(c);
     if (!st) st = cuda_check(cudaStreamSynchronize(c->stream), "schedule upload");
     if (st) return st;
     c->version += 1;
@@ -1326,6 +1354,8 @@ piks_status piks_autotune(piks_ctx *c, const int32_t *cand, int32_t ncand, int32
   cudaEventCreate(&e1);
   const bool timing = c->timing;
   c->timing = false;
+  const int32_t old[4] = {c->tile_dims[0], c->tile_dims[1], c->tile_dims[2], c->schedule};
+  const bool old_wave = c->use_wave;
   // makes candidate k the context's schedule (a column candidate ignores its tile shape)
   auto take = [c](const int32_t *k, bool *ok) -> piks_status {
     c->tile_dims[0] = k[0]; c->tile_dims[1] = k[1]; c->tile_dims[2] = k[2];
@@ -1334,9 +1364,7 @@ piks_status piks_autotune(piks_ctx *c, const int32_t *cand, int32_t ncand, int32
     c->use_tiles = false;
     c->use_wave = k[3] == PIKS_SCHED_WAVE && build_wave(c);
     *ok = c->use_wave || (k[3] != PIKS_SCHED_WAVE && build_tiles(c));
-    if (!*ok) return PIKS_OK;
-    const piks_status st = upload_wave(c);
-    return st ? st : upload_tiles(c);
+    return *ok ? upload_schedule(c) : PIKS_OK;
   };
   double best = 1e300;
   int bi = -1;
@@ -1365,28 +1393,23 @@ piks_status piks_autotune(piks_ctx *c, const int32_t *cand, int32_t ncand, int32
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c->timing = timing;
-  if (st) return st;
-  if (bi < 0) return fail(PIKS_ERR_ARG, "no usable tile candidate");
   const int32_t *k = cand + 4 * bi;
   bool ok = false;
-  if ((st = take(k, &ok))) return st;
-  c->tiles_tuned = true;
-  // the trial sweeps changed f: back to the state of setupFlow (all zero)
-  const StateSizes z = state_sizes(c);
-  DevState &s = c->ds;
-  const size_t e = c->prec == PIKS_PREC_FP32 ? sizeof(float) : sizeof(double);
-  void *hs = c->prec == PIKS_PREC_FP32 ? (void *)s.h32 : (void *)s.h;
-  void *fws = c->prec == PIKS_PREC_FP32 ? (void *)s.fw32 : (void *)s.fw;
-  cudaMemsetAsync(hs, 0, z.h * e, c->stream);
-  if (z.fw) cudaMemsetAsync(fws, 0, z.fw * e, c->stream);
-  for (int b = 0; b < 2; ++b) {
-    cudaMemsetAsync(c->prec == PIKS_PREC_FP32 ? (void *)s.ghostW32[b] : (void *)s.ghostW[b], 0, z.plane * e, c->stream);
-    cudaMemsetAsync(c->prec == PIKS_PREC_FP32 ? (void *)s.ghostE32[b] : (void *)s.ghostE[b], 0, z.plane * e, c->stream);
-  }
-  cudaMemsetAsync(s.mom, 0, (size_t)c->geo.NF * 4 * sizeof(double), c->stream);
+  if (!st && bi >= 0) st = take(k, &ok);
   c->version += 1;
+  if (st || bi < 0) {
+    // the schedule that the context had
+    const std::string why = st ? g_last_error : "no usable tile candidate";
+    std::copy(old, old + 3, c->tile_dims);
+    c->schedule = old[3];
+    build_schedule(c, old_wave);
+    piks_status back = upload_schedule(c);
+    if (!back) back = reset_state(c);
+    return back ? back : fail(st ? st : PIKS_ERR_ARG, why);
+  }
+  c->tiles_tuned = true;
   if (chosen) for (int j = 0; j < 4; ++j) chosen[j] = k[j];
-  return cuda_check(cudaStreamSynchronize(c->stream), "autotune reset");
+  return reset_state(c);  // the trial sweeps changed f
 }
 
 piks_status piks_get_precision(piks_ctx *c, int32_t *precision) {

@@ -55,3 +55,26 @@ def test_switching_schedules_keeps_the_iteration():
                     s.set_precision(pk.PREC_FP64)
             out.append((s.get_f()[0], s.chk_converge()))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("own", [None, (4, 4, 4), (0, 0, 0)])
+def test_autotune_without_a_usable_candidate_keeps_the_schedule(own):
+    """16^3 tiles of this box need more rows than shared memory holds. An autotune call that is given
+    nothing else reports that; the context then iterates on the schedule it had (columns, tiles or
+    nodes), from the state of a set-up, as one that was never tuned."""
+    img = images.sphere_pack(20, 0.45, 1.5, 3.0, seed=8)
+    p = base_params(20, Nc_fundamental=4, Kn=0.5, wallExtOrder=1)
+    out = []
+    for tune in (True, False):
+        with pk.Solver(p, device=0) as s:
+            if own:
+                s.set_tiles(*own)
+            s.setup_physical_grid(img)
+            before = s.schedule()
+            if tune:
+                with pytest.raises(pk.PiksError, match="candidate"):
+                    s.autotune([(16, 16, 16, pk.SCHED_TILE_DIAGONALS), (16, 16, 16, pk.SCHED_TILE_DATAFLOW)], sweeps=1)
+                assert s.schedule() == before
+            s.iterate(4)
+            out.append((s.get_f()[0], s.chk_converge()))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
