@@ -635,7 +635,10 @@ piks_status upload_tiles(piks_ctx *c) {
 piks_status upload_schedule(piks_ctx *c) {
   piks_status st = upload_wave(c);
   if (!st) st = upload_tiles(c);
-  if (st) c->use_wave = c->use_tiles = false;
+  if (st) {
+    c->use_wave = c->use_tiles = false;
+    c->version += 1;               // graphs and batches hold buffers that are gone
+  }
   return st;
 }
 
