@@ -265,8 +265,12 @@ piks_status piks_set_schedule(piks_ctx *ctx, int32_t schedule);
  * milliseconds per sweep of each candidate (-1 where a candidate does not apply). */
 piks_status piks_autotune(piks_ctx *ctx, const int32_t *candidates, int32_t ncand, int32_t sweeps,
                           int32_t *chosen, double *ms_out);
-/* [columns or tiles in use (0: the per-node schedule), TX, TY, TZ, largest shared-memory slot count of a job,
- *  launch schedule, number of jobs] */
+/* The sweep schedule in use, up to 11 entries: [columns or tiles (0: the per-node schedule),
+ * TX, TY, TZ, largest shared-memory slot count of a tile job, launch schedule, number of tile
+ * jobs, cross-section of the columns in x and y, rows of their ring, number of columns]. A
+ * context on the columns has no tile jobs (slots and jobs are 0 unless the tile_* arrays of
+ * piks_geometry_array were asked for) and reports the shape they would take; one on tiles or
+ * nodes has 0 in the last four. Before the first set-up the launch schedule is the one asked for. */
 piks_status piks_get_schedule(piks_ctx *ctx, int32_t *out, int32_t n);
 
 /* FP32 solve with FP64 refinement: runs FP32 iterations with chkConverge every

@@ -293,11 +293,12 @@ class Solver:
         return tuple(chosen), ms[:n]
 
     def schedule(self):
-        """{'tiles': bool, 'TX', 'TY', 'TZ', 'max_slots', 'launch', 'jobs'} of the sweep schedule."""
-        a = (ctypes.c_int32 * 7)()
-        _check(self.lib.piks_get_schedule(self._ctx, a, 7))
+        """{'tiles': bool, 'TX', 'TY', 'TZ', 'max_slots', 'launch', 'jobs', 'cross_section', 'ring',
+        'columns'} of the sweep schedule in use (piks_get_schedule)."""
+        a = (ctypes.c_int32 * 11)()
+        _check(self.lib.piks_get_schedule(self._ctx, a, 11))
         return {"tiles": bool(a[0]), "TX": a[1], "TY": a[2], "TZ": a[3], "max_slots": a[4], "launch": a[5],
-                "jobs": a[6]}
+                "jobs": a[6], "cross_section": (a[7], a[8]), "ring": a[9], "columns": a[10]}
 
     @property
     def precision(self):

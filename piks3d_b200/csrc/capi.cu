@@ -494,7 +494,7 @@ bool build_wave(piks_ctx *c) {
 }
 
 // The tile jobs of a context that iterates the hyperplane columns, built for the calls that
-// report or use them.
+// use them.
 void ensure_tiles(piks_ctx *c) {
   if (c->use_wave && c->tiles.row_count.empty() && c->tile_dims[0] > 0)
     build_tiles_for(c, c->tile_dims, TILE_FORM_SLOTS, c->tiles, c->prec);
@@ -1334,10 +1334,19 @@ piks_status piks_set_schedule(piks_ctx *c, int32_t schedule) {
 
 piks_status piks_get_schedule(piks_ctx *c, int32_t *out, int32_t n) {
   if (!c || !out) return fail(PIKS_ERR_ARG, "null argument");
-  ensure_tiles(c);
-  const int32_t v[7] = {c->use_tiles || c->use_wave ? 1 : 0, c->tiles.TX, c->tiles.TY, c->tiles.TZ, c->tiles.max_rows,
-                        c->schedule, (int32_t)c->tiles.row_count.size()};
-  for (int i = 0; i < n && i < 7; ++i) out[i] = v[i];
+  // what the context iterates: a schedule asked for since takes effect at the next set-up, and
+  // one that does not fit falls back
+  int32_t launch = c->schedule;
+  if (c->use_wave) launch = PIKS_SCHED_WAVE;
+  else if (c->have_host_geometry && launch == PIKS_SCHED_WAVE) launch = PIKS_SCHED_TILE_DIAGONALS;
+  const bool built = !c->use_wave || !c->tiles.row_count.empty();
+  const int32_t v[11] = {c->use_tiles || c->use_wave ? 1 : 0,
+                         built ? c->tiles.TX : c->tile_dims[0], built ? c->tiles.TY : c->tile_dims[1],
+                         built ? c->tiles.TZ : c->tile_dims[2], c->tiles.max_rows, launch,
+                         (int32_t)c->tiles.row_count.size(),
+                         c->use_wave ? c->wave.A : 0, c->use_wave ? c->wave.B : 0, c->use_wave ? c->wave.ring : 0,
+                         c->use_wave ? c->wave.ncol : 0};
+  for (int i = 0; i < n && i < 11; ++i) out[i] = v[i];
   return PIKS_OK;
 }
 

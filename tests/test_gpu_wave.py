@@ -8,7 +8,9 @@ import pytest
 
 import piks3d_b200 as pk
 from conftest import base_params
+from oracle import SlabOracle
 from piks3d_b200 import images
+from piks3d_b200.slab import LocalSlabs
 
 pytestmark = pytest.mark.gpu
 
@@ -78,3 +80,41 @@ def test_autotune_without_a_usable_candidate_keeps_the_schedule(own):
             s.iterate(4)
             out.append((s.get_f()[0], s.chk_converge()))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+def test_tile_diagonals_by_name_move_to_the_fp64_shape():
+    """Tile diagonals asked for by name, without a shape: FP32 tiles of 4x4x4 that move to 8x4x4 at
+    the switch to FP64 and give the columns' values."""
+    img = images.sphere_pack(16, 0.5, 1.5, 3.5, seed=1)
+    p = base_params(16, Nc_fundamental=4, Kn=0.5, fluidlayer=2)
+    out = []
+    for sched in (pk.SCHED_TILE_DIAGONALS, pk.SCHED_WAVE):
+        with pk.Solver(p, device=0) as s:
+            s.set_schedule(sched)
+            s.set_precision(pk.PREC_FP32)
+            s.setup_physical_grid(img)
+            assert s.schedule()["launch"] == sched and s.schedule()["TX"] == 4
+            s.iterate(6)
+            s.set_precision(pk.PREC_FP64)
+            assert s.schedule()["launch"] == sched and s.schedule()["TX"] == 8
+            s.iterate(5)
+            out.append((s.get_f()[0], s.chk_converge()))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("sched", [pk.SCHED_TILE_DIAGONALS, pk.SCHED_WAVE])
+@pytest.mark.parametrize("n", [2, 3])
+def test_slabs_by_schedule_equal_the_slab_oracle(n, sched):
+    img = images.sphere_pack(16, 0.45, 1.2, 3.0, seed=2)
+    p = base_params(16, wallExtOrder=1, Nc_fundamental=4)
+    ls = LocalSlabs(p, img, n, schedule=sched)
+    so = SlabOracle(p, img.tobytes(), n, nthreads=8)
+    assert all(s.schedule()["launch"] == sched and s.schedule()["tiles"] for s in ls.solvers)
+    for _ in range(3):
+        ls.iterate(1)
+        so.iterate(1)
+    for a, b in zip(so.macro(), ls.macro()):
+        assert np.array_equal(a, b)
+    assert ls.chk_converge() == so.chk_converge()
+    ls.close()
+    so.close()

@@ -109,3 +109,25 @@ def test_warps_that_may_leave_meet_on_mbarriers_only():
     assert counted == ["__syncthreads"]
     kernel = code[code.index("k_wave_sweep(const DevState a"):]
     assert kernel.index("__syncthreads") < kernel.index("setmaxnreg")
+
+
+def test_schedule_reports_what_is_in_use():
+    """The getter describes the schedule that the context iterates and builds nothing: no tile jobs
+    on a context that marches columns, and no column schedule named where another one runs."""
+    img = images.sphere_pack(24, 0.5, 1.5, 3.5, seed=4)
+    s = pk.Solver(base_params(24), device=-1)
+    s.setup_physical_grid(img)
+    sch = s.schedule()
+    A, B, ring = s.geometry_array("wave_info").tolist()[:3]
+    assert sch["launch"] == pk.SCHED_WAVE and sch["tiles"] and sch["jobs"] == 0 and sch["max_slots"] == 0
+    assert (sch["cross_section"], sch["ring"], sch["columns"]) == ((A, B), ring, len(s.geometry_array("wave_cols")) // 8)
+    s.set_tiles(4, 4, 4)                         # from the next set-up on
+    assert s.schedule()["launch"] == pk.SCHED_WAVE and s.schedule()["columns"] == sch["columns"]
+    s.setup_physical_grid(img)
+    sch = s.schedule()
+    assert sch["launch"] == pk.SCHED_TILE_DIAGONALS and sch["jobs"] > 0 and (sch["cross_section"], sch["columns"]) == ((0, 0), 0)
+    s.close()
+    s = pk.Solver(base_params(12), device=-1)
+    s.setup_physical_grid(np.ones((12, 12, 12), np.uint8))   # nothing to sweep: no columns are built
+    assert s.schedule()["launch"] != pk.SCHED_WAVE and s.schedule()["columns"] == 0
+    s.close()
