@@ -208,13 +208,16 @@ piks_status piks_selftest_division(int32_t device, int64_t samples, uint64_t see
  * Has no counterpart in the reference, which has no device code. */
 piks_status piks_selftest_division_noalloc(int32_t device, int64_t samples, uint64_t seed, int64_t *mismatches);
 
-/* Self-test of the bounded waits of the dataflow sweep: runs one tile-dataflow sweep of
- * the context in which one job waits on a flag that no job sets. Its wait gives up after
- * its iteration limit (about a second), sets the sweep's error flag, and every job finishes;
- * the call restores the schedule, clears the flag, and stores the sweep's duration in
- * *seconds. Returns PIKS_OK when the wait ran out as designed, PIKS_ERR_STATE when it did not
- * (or the context has no tile schedule). The sweep overwrites f with values that are not the
- * solver's: set the image up again before iterating. Has no counterpart in the reference. */
+/* Self-test of the bounded waits of a sweep. On a context that marches columns: one column
+ * sweep in which a column waits for a hyperplane that no column publishes, alone and in a batch
+ * of one; on tiles: one tile-dataflow sweep in which a job waits on a flag that no job sets. The
+ * wait gives up after its limit (one to two seconds) and sets the sweep's error flag, which
+ * piks_synchronize and the convergence checks report; the call restores the schedule, clears the
+ * flag, and stores the (first) sweep's duration in *seconds. Returns PIKS_OK when the waits ran
+ * out as designed, PIKS_ERR_STATE when one did not, or when the context iterates neither form or
+ * its image has one column an octant. The sweep overwrites f with values that are not the
+ * solver's: set the image up again before iterating. Not while the context is in a batch. Has
+ * no counterpart in the reference. */
 piks_status piks_selftest_wait_timeout(piks_ctx *ctx, double *seconds);
 
 /* Storage and sweep precision of a context. PIKS_PREC_FP64 (the default) is the

@@ -310,8 +310,9 @@ class Solver:
         _check(self.lib.piks_synchronize(self._ctx))
 
     def selftest_wait_timeout(self):
-        """Runs one dataflow sweep in which a job waits on a flag nothing sets; returns the
-        sweep's duration (s) once the wait has given up as designed (piks_selftest_wait_timeout).
+        """Runs one sweep of the columns (or of the tile dataflow) in which a column (a job) waits for
+        what nothing publishes; returns the sweep's duration (s) once the wait has given up as
+        designed (piks_selftest_wait_timeout).
         The state's values are not the solver's afterwards: set the image up again."""
         sec = ctypes.c_double()
         _check(self.lib.piks_selftest_wait_timeout(self._ctx, ctypes.byref(sec)))

@@ -106,7 +106,7 @@ piks_status rebuild(piks_batch *b) {
   for (size_t m = 0; m < nm; ++m) hs[m] = b->members[m]->ds;
   size_t prog = kMaxClasses;
   for (size_t m = 0; m < nm; ++m)
-    if (b->members[m]->use_wave) prog += (size_t)hs[m].wv.ncol * hs[m].wv.nchunk;
+    if (b->members[m]->use_wave) prog += (size_t)(hs[m].wv.ncol + 1) * hs[m].wv.nchunk;
   if (prog > b->prog_cap) {
     if (b->d_prog) cudaFree(b->d_prog);
     b->d_prog = nullptr;
@@ -120,7 +120,7 @@ piks_status rebuild(piks_batch *b) {
   for (size_t m = 0; m < nm; ++m)
     if (b->members[m]->use_wave) {
       hs[m].wv.progress = b->d_prog + prog;
-      prog += (size_t)hs[m].wv.ncol * hs[m].wv.nchunk;
+      prog += (size_t)(hs[m].wv.ncol + 1) * hs[m].wv.nchunk;
     }
   if (nm) {
     piks_status st = cuda_check(cudaMemcpyAsync(b->d_states, hs.data(), nm * sizeof(DevState), cudaMemcpyHostToDevice,

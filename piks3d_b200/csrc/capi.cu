@@ -555,10 +555,11 @@ piks_status upload_wave(piks_ctx *c) {
     if ((st = upload(c, items, &c->wave_items[f32]))) return st;
   }
   int *pw = nullptr;
-  if ((st = zeros(c, (size_t)wj.ncol * most + 8, &pw))) return st;
+  // one more column's worth of progress than columns: that column never publishes (wait self-test)
+  if ((st = zeros(c, (size_t)(wj.ncol + 1) * most + 8, &pw))) return st;
   w.counter = pw;                 // the progress array follows it, the error flag comes last
   w.progress = pw + 4;
-  w.err = pw + 4 + (size_t)wj.ncol * most;
+  w.err = pw + 4 + (size_t)(wj.ncol + 1) * most;
   w.ncol = wj.ncol;
   w.A = wj.A; w.B = wj.B;
   w.ring = wj.ring; w.task_ring = wj.task_ring; w.max_rows = wj.max_rows;
@@ -1783,18 +1784,52 @@ piks_status piks_launches_per_iteration(piks_ctx *c, int64_t *n) {
   return PIKS_OK;
 }
 
+// The wait self-test of a context on the columns: a column with rows of an upwind column waits
+// for one that does not exist, in a sweep of the context and in one of a batch that holds it.
+static piks_status selftest_wave_wait(piks_ctx *c, double *seconds) {
+  cudaSetDevice(c->device);
+  const WaveJobs &wj = c->wave;
+  int col = -1;
+  for (int k = 0; k < wj.ncol && col < 0; ++k) {
+    const int32_t *h = &wj.cols[(size_t)k * 8], *b = &wj.batch[(size_t)h[0] * 4];
+    for (int i = 0; i < h[1] && col < 0; ++i)
+      if ((b[4 * i + 3] & 0xFFFF) < (b[4 * i + 2] & 0xFFFF)) col = k;
+  }
+  if (col < 0) return fail(PIKS_ERR_STATE, "no column of this image waits for another");
+  // (entry 4 of a column's record: the column upwind in x)
+  int32_t *up = reinterpret_cast<int32_t *>(const_cast<int4 *>(c->ds.wv.cols)) + (size_t)col * 8 + 4;
+  const int32_t old_up = wj.cols[(size_t)col * 8 + 4], never = wj.ncol;
+  piks_status st = cuda_check(cudaStreamSynchronize(c->stream), "selftest sync");
+  if (!st) st = cuda_check(cudaMemcpy(up, &never, sizeof(int32_t), cudaMemcpyHostToDevice), "selftest up");
+  if (st) return st;
+  const auto t0 = std::chrono::steady_clock::now();
+  launch_wave_sweep(c->ds, c->prec == PIKS_PREC_FP32, c->stream);
+  st = cuda_check(cudaStreamSynchronize(c->stream), "selftest sweep");
+  *seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  const bool alone = !st && check_sweep_error(c) != PIKS_OK;
+  bool batched = false;
+  if (!st) {
+    piks_batch *b = nullptr;
+    st = piks_batch_create(c->device, &b);
+    if (!st) st = piks_batch_add(b, c);
+    if (!st) st = piks_batch_iterate(b, 1);
+    if (!st) st = piks_batch_synchronize(b);
+    if (!st) batched = piks_batch_chk_converge(b, nullptr, nullptr, nullptr) != PIKS_OK;
+    piks_batch_destroy(b);
+  }
+  // restore the schedule and clear the error flag in any case
+  cudaMemcpy(up, &old_up, sizeof(int32_t), cudaMemcpyHostToDevice);
+  cudaMemset(c->ds.wv.err, 0, sizeof(int));
+  if (st) return st;
+  if (!alone || !batched) return fail(PIKS_ERR_STATE, alone ? "the batch's column wait did not give up" : "the column wait did not give up");
+  return PIKS_OK;
+}
+
 piks_status piks_selftest_wait_timeout(piks_ctx *c, double *seconds) {
   if (!c || !seconds) return fail(PIKS_ERR_ARG, "null argument");
-  if (c->device >= 0 && c->have_geometry && c->use_wave && c->ds.tv.njobs < 1) {
-    // a context that iterates the columns runs the self-test on its tile jobs
-    cudaSetDevice(c->device);
-    ensure_tiles(c);
-    piks_status st = upload_tiles(c);
-    if (!st) st = cuda_check(cudaStreamSynchronize(c->stream), "selftest tiles");
-    if (st) return st;
-  }
-  if (c->device < 0 || !c->have_geometry || !(c->use_tiles || c->use_wave) || c->ds.tv.njobs < 1 || c->tiles.split)
-    return fail(PIKS_ERR_STATE, "the wait self-test needs a device state with a dataflow or diagonal tile schedule");
+  if (c->device >= 0 && c->have_geometry && c->use_wave) return selftest_wave_wait(c, seconds);
+  if (c->device < 0 || !c->have_geometry || !c->use_tiles || c->ds.tv.njobs < 1 || c->tiles.split)
+    return fail(PIKS_ERR_STATE, "the wait self-test needs a device state with a column, dataflow or diagonal schedule");
   cudaSetDevice(c->device);
   DevState &s = c->ds;
   TileView &tv = s.tv;

@@ -36,7 +36,7 @@ struct WaveView {
   const int4 *batch;            // row group (of 4), first task, rows | tasks << 16, own + static rows | ring slot << 16
   const int4 *cols;             // [ncol][2]: first batch, batches, octant, first local hyperplane | upwind columns in x, y (or -1)
   const int4 *items;            // (0, column, chunk, 0) in dependency order
-  int *progress;                // [ncol][nchunk] hyperplanes done, cleared before each sweep
+  int *progress;                // [ncol + 1][nchunk] hyperplanes done, cleared before each sweep
   int *counter;                 // item counter, cleared with the progress array behind it
   int *err;                     // set when a wait gave up
   int ncol, nchunk, A, B;       // columns, velocity chunks, cross-section of a column

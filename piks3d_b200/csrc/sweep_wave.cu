@@ -838,7 +838,7 @@ int wave_max_ring(int Nc8, bool fp32, int task_ring, int max_rows) {
 
 void launch_wave_sweep(const DevState &s, bool fp32, cudaStream_t st) {
   const WaveView &w = s.wv;
-  cudaMemsetAsync(w.counter, 0, ((size_t)w.ncol * w.nchunk + 4) * sizeof(int), st);
+  cudaMemsetAsync(w.counter, 0, ((size_t)(w.ncol + 1) * w.nchunk + 4) * sizeof(int), st);
   launch_wave_any<false>(s, nullptr, w.items, w.ncol * w.nchunk, fp32, wave_velocities(s.Nc8, fp32),
                          {w.ring, w.task_ring, w.max_rows}, w.counter, w.err, st);
 }

@@ -118,3 +118,39 @@ def test_slabs_by_schedule_equal_the_slab_oracle(n, sched):
     assert ls.chk_converge() == so.chk_converge()
     ls.close()
     so.close()
+
+
+@pytest.mark.parametrize("nf,prec", [(4, pk.PREC_FP64), (4, pk.PREC_FP32), (2, pk.PREC_FP32)])
+def test_column_waits_give_up_and_the_context_stays_usable(nf, prec):
+    """A column that waits for a hyperplane nobody publishes (no fault, trap or hang): its wait runs
+    out, alone and in a batch, the sweep ends with the error reported, and the context, set up
+    again, iterates as a fresh one. 512 velocities: two chunks an octant in FP64, so that the
+    consumers change their class table on the way."""
+    img = images.sphere_pack(33, 0.6, 1.5, 3.5, seed=9)
+    p = base_params(33, Nc_fundamental=nf, Kn=0.8, wallExtOrder=1)
+    with pk.Solver(p, device=0) as s:
+        s.set_precision(prec)
+        s.setup_physical_grid(img)
+        assert s.schedule()["launch"] == pk.SCHED_WAVE and s.schedule()["columns"] > 8
+        s.iterate(3)
+        sec = s.selftest_wait_timeout()
+        print("column sweep with a wait that nothing ends: %.3f s" % sec)
+        assert 0.5 < sec < 10.0
+        s.synchronize()
+        s.setup_physical_grid(img)
+        s.iterate(5)
+        a = (s.get_f()[0], s.chk_converge())
+    with pk.Solver(p, device=0) as r:
+        r.set_precision(prec)
+        r.setup_physical_grid(img)
+        r.iterate(5)
+        b = (r.get_f()[0], r.chk_converge())
+    assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+
+
+def test_wait_selftest_refuses_a_box_of_one_column():
+    img = images.sphere_pack(8, 0.6, 1.2, 2.5, seed=9)
+    with pk.Solver(base_params(8, Nc_fundamental=4), device=0) as s:
+        s.setup_physical_grid(img)
+        with pytest.raises(pk.PiksError, match="waits for another"):
+            s.selftest_wait_timeout()
