@@ -331,6 +331,13 @@ piks_status check_sweep_error(piks_ctx *c) {
   return PIKS_OK;
 }
 
+// Wall launches of an iteration: one per dependency level, or one for all walls where every wall
+// extrapolates from its first point only and reads no other.
+size_t wall_launches(const piks_ctx *c) {
+  const auto &ls = c->geo.level_start;
+  return ls.empty() ? 0 : c->ds.wall_far ? ls.size() - 1 : std::min<size_t>(ls.size() - 1, 1);
+}
+
 // The boundary part of iteration n (solver.F90:535-1938): switch commits, halo capture,
 // walls, inlet/outlet, symmetry, moments, on stream st.
 void enqueue_boundaries_timed(piks_ctx *c, cudaStream_t st, int n) {
@@ -346,9 +353,7 @@ void enqueue_boundaries_timed(piks_ctx *c, cudaStream_t st, int n) {
   {
     Timed t(c, KT_WALLS);
     const auto &ls = c->geo.level_start;
-    // (walls that extrapolate from their first point only read no other wall: one launch)
-    const size_t n = ls.empty() ? 0 : s.wall_far ? ls.size() - 1 : std::min<size_t>(ls.size() - 1, 1);
-    for (size_t L = 0; L < n; ++L) {
+    for (size_t L = 0, n = wall_launches(c); L < n; ++L) {
       const int end = s.wall_far ? ls[L + 1] : ls.back();
       if (f32) launch_walls32(s, ls[L], end, prev, st);
       else launch_walls(s, ls[L], end, prev, st);
@@ -1778,7 +1783,7 @@ piks_status piks_launches_per_iteration(piks_ctx *c, int64_t *n) {
   } else {
     for (size_t h = 0; h + 1 < c->geo.hyper_start.size(); ++h) k += c->geo.hyper_start[h + 1] > c->geo.hyper_start[h];
   }
-  k += (s.ncommit > 0) + 1 /*capture*/ + (int64_t)(c->geo.level_start.size() - 1) + 1 /*inlet*/ +
+  k += (s.ncommit > 0) + 1 /*capture*/ + (int64_t)wall_launches(c) + 1 /*inlet*/ +
        (s.nsym > 0) + (s.NF > 0);
   *n = k;
   return PIKS_OK;

@@ -65,3 +65,14 @@ def test_fp32_walls_and_moments(nf, order):
             terms = np.array(signs)[:, None, None] * c[None, :, None] * fluid
             bound = 2 * 8 * nc8 * 2.0 ** -53 * np.abs(terms).sum(axis=(0, 1))
             assert np.all(np.abs(got.ravel()[at] - terms.sum(axis=(0, 1))) <= bound)
+
+
+def test_wall_launches_are_counted_as_launched():
+    """Walls that read their first extrapolation point only are one launch, others one per level."""
+    img = images.sphere_pack(16, 0.45, 1.2, 3.0, seed=5)
+    n = {}
+    for order in (1, 2):
+        with pk.Solver(base_params(16, wallExtOrder=order), device=0) as s:
+            s.setup_physical_grid(img)
+            n[order], levels = s.launches_per_iteration(), s.info()["nWallLevels"]
+    assert levels > 1 and n[2] - n[1] == levels - 1
