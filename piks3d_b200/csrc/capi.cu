@@ -9,7 +9,9 @@
 #include <cstdio>
 #include <cstring>
 #include <future>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -99,14 +101,14 @@ void release(piks_ctx *c, void *p) {
 }
 
 // Pinned slices for fetch_macro, kept between calls while some device context lives: a call
-// borrows a stage (the first of a process takes 2 to 3 ms to allocate), at most two wait here,
-// of at most 16 slices of 256 KiB each.
+// borrows a stage, at most two wait here, of at most 16 slices of 256 KiB each.
 struct MacroStage { double *p; int slices; };
 struct StagePool {
   std::mutex lock;
   std::vector<MacroStage> idle;
   int contexts = 0;
-  MacroStage take(int slices, size_t slice) {
+  // An idle stage, or (where `allocate`) a new one; p is null when there is none.
+  MacroStage take(int slices, size_t slice, bool allocate) {
     {
       std::lock_guard<std::mutex> hold(lock);
       for (size_t i = 0; i < idle.size(); ++i)
@@ -117,7 +119,7 @@ struct StagePool {
         }
     }
     MacroStage s{nullptr, slices};
-    if (cudaMallocHost(&s.p, slice * slices * sizeof(double)) != cudaSuccess) {
+    if (allocate && cudaMallocHost(&s.p, slice * slices * sizeof(double)) != cudaSuccess) {
       (void)cudaGetLastError();
       s.p = nullptr;
     }
@@ -150,7 +152,12 @@ StagePool g_macro_stages;
 // and for its own copies. What bounds it is
 // the first touch of the caller's pages. One thread, a whole pageable copy and four passes over
 // the box took 1.1 / 2.2 / 50 / 250 ms for boxes of 32^3 / 48^3 / 128^3 / 256^3 voxels; this takes
-// 0.25 / 0.45 / 3 / 18 ms on 16 cores (a process's first call allocates the slices: 2 to 3 ms more).
+// 0.25 / 0.45 / 3 / 18 ms on 16 cores with pinned slices at hand.
+// A context's first call allocates them only for eight blocks a thread or more: a program that
+// solves one image a context fetches its fields once, and 16 slices take 4 to 6 ms to pin. First
+// call of a context, pinned on demand / pageable, porosity 0.45: 32^3 3.0 / 0.33 ms, 48^3 2.7 / 0.98,
+// 96^3 5.8 / 3.2, 128^3 (115 blocks, 16 threads) 9.7 / 9.1, 160^3 12.2 / 16.7, 192^3 17 / 27; later
+// calls 48^3 0.45 / 1.0, 128^3 4.1 / 9.0.
 constexpr int64_t kMacroNodes = 8192;
 cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
   const Geometry &g = c->geo;
@@ -158,12 +165,14 @@ cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
   const unsigned hw = std::thread::hardware_concurrency();
   const int nw = (int)std::min<int64_t>(std::max(1u, std::min(hw ? hw : 1u, 16u)), nblock);
   const size_t slice = (size_t)kMacroNodes * 4;
-  const MacroStage pinned = g_macro_stages.take(nw, slice);
-  std::vector<double> pageable;
+  const MacroStage pinned = g_macro_stages.take(nw, slice, c->macro_calls > 0 || nblock >= 8 * nw);
+  c->macro_calls = 1;
+  std::unique_ptr<double[]> pageable;
   if (!pinned.p) {
-    try { pageable.resize(slice * nw); } catch (const std::bad_alloc &) { return cudaErrorMemoryAllocation; }
+    pageable.reset(new (std::nothrow) double[slice * nw]);
+    if (!pageable) return cudaErrorMemoryAllocation;
   }
-  double *stage = pinned.p ? pinned.p : pageable.data();
+  double *stage = pinned.p ? pinned.p : pageable.get();
   const int64_t box = (int64_t)g.Nx * g.Ny * g.Nz;
   auto voxel = [&](int64_t n) -> int64_t {
     const uint32_t gi = (uint32_t)g.node_g[(size_t)n], gx = (uint32_t)g.GX, gy = (uint32_t)g.GY;

@@ -47,6 +47,7 @@ struct piks_ctx {
   int prep = PIKS_PREP_DEVICE;      // where voxels are classified (device contexts)
   double setup_seconds[4] = {0, 0, 0, 0};  // last setup: box, classification, rest of the geometry, all
   int iStep = 0;
+  int macro_calls = 0;              // fields fetched before (fetch_macro's staging)
   int version = 0;                  // bumped whenever the device state is reallocated
   // copies of the iteration state (piks_snapshot_slot): per slot f, fw, moments and the
   // ghost planes the next iteration reads, slots back to back in one buffer

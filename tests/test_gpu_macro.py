@@ -36,3 +36,17 @@ def test_fields_wait_for_the_iterations_of_the_callers_stream(edge, stream):
     assert any(np.any(w) for w in want)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("edge", [16, 40])
+def test_fields_are_the_same_on_every_call(edge):
+    """The first call of a context stages a small box in pageable memory, later ones in pinned."""
+    img = images.sphere_pack(edge, 0.7, 2.0, 4.0, seed=6)
+    with pk.Solver(base_params(edge, wallExtOrder=1), device=0) as s:
+        s.setup_physical_grid(img)
+        s.iterate(12)
+        first, rest = s.get_macro(), [s.get_macro() for _ in range(3)]
+        assert any(np.any(f) for f in first)
+        for got in rest:
+            for a, b in zip(got, first):
+                assert np.array_equal(a, b)
