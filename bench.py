@@ -487,7 +487,7 @@ def small_batch(args, world, rank, local, device):
                                 "converged": sum(1 for r in by.values() if r["converged"])},
             "speedup_solves_per_s": t_plain / t_batch,
             "perm_rel_diff_refined_vs_fp64": {"max": max(diffs), "median": float(np.median(diffs))},
-            "autotuned_tiles": sorted({str(r.get("tiles")) for r in by.values()})}
+            "schedules": sorted({r["schedule"] for r in by.values() if "schedule" in r})}
 
 
 def run_batch_workload(args, world, rank, local):

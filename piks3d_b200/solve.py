@@ -21,7 +21,7 @@ import time
 
 import numpy as np
 
-from . import Batch, PREC_FP32, PREC_FP64, SCHED_WAVE, Solver
+from . import Batch, PREC_FP32, PREC_FP64, Solver
 
 
 class Convergence:
@@ -188,7 +188,7 @@ class Job:
         self.image, self.params, self.name, self.arrival = image, params, name, arrival
         self.make_image, self.porosity = make_image, porosity
         self.solver = None
-        self.tuned = None             # (TX, TY, TZ, schedule) chosen by the batch runner's autotuner
+        self.tuned = None             # (TX, TY, TZ, schedule) chosen by the batch runner's autotuner, if it timed any
         self.conv = None
         self.ex = None                # Extrapolator of a refined job's FP32 phase
         self.phase = None             # "fp32" / "fp64"
@@ -228,11 +228,11 @@ def footprint_bytes(image, params, precision="refined", slots=None):
     return max((f32 + moments) * (1 + slots), f32 + f64 + moments) + tables
 
 
-# Schedules the batch runner's autotuner times on each job. The hyperplane columns, which a
-# context starts with, were the fastest at every size measured (8^3 to 96^3, 64 and 512
-# velocities, both precisions: 1.2 to 2.4 times the tile dataflow's sweep), so the list holds
-# only them and nothing is timed.
-TUNE_CANDIDATES = ((8, 4, 4, SCHED_WAVE),)
+# Schedules, (TX, TY, TZ, launch) each, that the batch runner's autotuner times on each job. The
+# hyperplane columns, which a context starts with, were the fastest at every size measured (8^3
+# to 96^3, 64 and 512 velocities, both precisions: 1.2 to 2.4 times the tile dataflow's sweep),
+# so the list is empty and nothing is timed; a program may set its own.
+TUNE_CANDIDATES = ()
 
 
 def _prepare(job, device, precision, autotune=False):
@@ -243,9 +243,7 @@ def _prepare(job, device, precision, autotune=False):
         if precision in ("fp32", "refined"):
             s.set_precision(PREC_FP32)
         s.setup_physical_grid(job.image)
-        if autotune and len(TUNE_CANDIDATES) == 1:
-            job.tuned = TUNE_CANDIDATES[0]
-        elif autotune:
+        if autotune and TUNE_CANDIDATES:
             # times one sweep of each candidate on this image (its own stream: the batch's
             # iterations may run meanwhile), keeps the fastest, resets the state
             job.tuned = s.autotune(TUNE_CANDIDATES, sweeps=1)[0]
@@ -258,7 +256,7 @@ def _prepare(job, device, precision, autotune=False):
 class BatchRunner:
     """Solves many jobs on one GPU as a continuously refilled batch: jobs are admitted while
     their estimated footprint fits the HBM budget and the batch has a free slot, preprocessed
-    (and, with `autotune`, their tile shape timed on the image) on host threads while the GPU
+    (and, with `autotune`, the schedules of TUNE_CANDIDATES timed on the image) on host threads while the GPU
     iterates, iterated together (piks_batch_*), checked every
     chkConvergeStep iterations, switched from FP32 to FP64 when their FP32 phase ends, and
     retired (state freed) as soon as they converge."""
@@ -385,6 +383,7 @@ class BatchRunner:
                               "permeability": float(perm[i]), "error": float(err[i]),
                               "converged": bool(conv), "diverged": job.conv.diverged,
                               "estimate": job.conv.estimate, "tiles": job.tuned,
+                              "schedule": job.solver.schedule()["launch"],
                               "jumps": job.ex.jumps if job.ex else 0}
                 if self.keep_fields:
                     job.result["macro"] = job.solver.get_macro()

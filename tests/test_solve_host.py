@@ -4,6 +4,7 @@ footprint estimate, and the request server's queueing, admission and latency acc
 import math
 
 import numpy as np
+import pytest
 
 import piks3d_b200 as pk
 from piks3d_b200.solve import Convergence, Job, footprint_bytes
@@ -359,3 +360,36 @@ def test_refinement_phase_uses_the_measured_contraction():
     j_fresh, m_fresh = run(None)
     assert abs(m_prior - limit) / limit <= tol and abs(m_fresh - limit) / limit <= tol
     assert j_prior < j_fresh
+
+
+class _TunedSolver:
+    """A Solver stand-in that records what the batch runner's preparation asks of it."""
+    def __init__(self, params, device=0):
+        self.asked = []
+
+    def set_precision(self, precision):
+        pass
+
+    def setup_physical_grid(self, image):
+        pass
+
+    def autotune(self, candidates, sweeps):
+        self.asked.append((tuple(candidates), sweeps))
+        return candidates[-1], [1.0] * len(candidates)
+
+
+@pytest.mark.parametrize("candidates", [(), ((8, 4, 4, 4),), ((4, 4, 4, 0), (8, 4, 4, 4))])
+def test_a_job_is_tuned_only_where_schedules_were_timed(monkeypatch, candidates):
+    """`tuned` names a schedule that the tuner timed on the job; with no candidates, or with the
+    tuner off, nothing is timed and nothing is reported."""
+    from piks3d_b200 import solve
+    monkeypatch.setattr(solve, "Solver", _TunedSolver)
+    assert solve.TUNE_CANDIDATES == ()           # the columns, which a context starts with, stand
+    monkeypatch.setattr(solve, "TUNE_CANDIDATES", candidates)
+    p = pk.default_params(Nx=8, Ny=8, Nz=8, Nc_fundamental=2)
+    job = Job(np.zeros((8, 8, 8), np.uint8), p)
+    s = solve._prepare(job, 0, "refined", autotune=True)
+    assert s.asked == ([(candidates, 1)] if candidates else [])
+    assert job.tuned == (candidates[-1] if candidates else None)
+    job = Job(np.zeros((8, 8, 8), np.uint8), p)
+    assert solve._prepare(job, 0, "refined", autotune=False).asked == [] and job.tuned is None
