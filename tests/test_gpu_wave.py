@@ -154,3 +154,80 @@ def test_wait_selftest_refuses_a_box_of_one_column():
         s.setup_physical_grid(img)
         with pytest.raises(pk.PiksError, match="waits for another"):
             s.selftest_wait_timeout()
+
+
+def _diagonal_plates(n):
+    """Solid and fluid plates of five cells each across one octant's direction: a whole hyperplane of
+    a column becomes fluid at once behind a solid one, and its tasks read most rows (the ring holds
+    685 rows beside the longer lists, 686 in every ordinary image, and a window of three batches 680)."""
+    i = np.indices((n, n, n))
+    return (((i.sum(0) + 3) % 10) < 5).astype(np.uint8)
+
+
+def _run(img, prec, steps, nodes=False, **kw):
+    with pk.Solver(base_params(img.shape[0], Kn=0.6, wallExtOrder=1, **kw), device=0) as s:
+        s.set_precision(prec)
+        if nodes:
+            s.set_tiles(*((0, 0, 0) if prec == pk.PREC_FP64 else (4, 4, 4)))
+        s.setup_physical_grid(img)
+        assert (s.schedule()["launch"] == pk.SCHED_WAVE) == (not nodes)
+        s.iterate(steps)
+        return s.get_f()[0], s.chk_converge(), s.schedule()["ring"]
+
+
+@pytest.mark.parametrize("prec", [pk.PREC_FP64, pk.PREC_FP32])
+def test_batch_of_members_with_different_rings(prec):
+    """Members whose rings differ: in FP32 one launch holds both and changes the ring between items,
+    in FP64 they go to launches of their own. Every member equals its run alone, which equals the
+    other schedule's."""
+    imgs = [images.sphere_pack(24, 0.5, 1.5, 3.5, seed=7), _diagonal_plates(24), images.sphere_pack(21, 0.6, 1.5, 3.0, seed=8)]
+    alone = [_run(i, prec, 4, Nc_fundamental=4) for i in imgs]
+    assert len({a[2] for a in alone}) == 2
+    other = _run(imgs[1], prec, 4, nodes=True, Nc_fundamental=4)
+    assert np.array_equal(alone[1][0], other[0]) and alone[1][1] == other[1]
+    members = []
+    with pk.Batch(device=0) as b:
+        for img in imgs:
+            s = pk.Solver(base_params(img.shape[0], Kn=0.6, wallExtOrder=1, Nc_fundamental=4), device=0)
+            s.set_precision(prec)
+            s.setup_physical_grid(img)
+            members.append(s)
+            b.add(s)
+        b.iterate(4)
+        mass, perm, err = b.chk_converge()
+    for k, s in enumerate(members):
+        assert np.array_equal(s.get_f()[0], alone[k][0]) and (mass[k], perm[k], err[k]) == alone[k][1]
+        s.close()
+
+
+@pytest.mark.parametrize("prec", [pk.PREC_FP64, pk.PREC_FP32])
+@pytest.mark.parametrize("nf", [8, 12, 16])
+def test_columns_of_many_velocity_chunks(nf, prec):
+    """Octants of 512, 1728 and 4096 velocities, up to 128 chunks a column, in a box of several columns."""
+    img = images.sphere_pack(14, 0.6, 1.2, 2.5, seed=21)[:7, :14, :14]
+    out = []
+    for wave in (True, False):
+        with pk.Solver(base_params(14, Nz=7, Nc_fundamental=nf, Kn=2.0, wallExtOrder=1), device=0) as s:
+            s.set_precision(prec)
+            if not wave:
+                s.set_tiles(*((0, 0, 0) if prec == pk.PREC_FP64 else (4, 4, 4)))
+            s.setup_physical_grid(img)
+            s.iterate(2)
+            out.append((s.get_f()[0], s.chk_converge(), s.schedule()["columns"]))
+    assert out[0][2] > 8 and out[1][2] == 0
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("prec", [pk.PREC_FP64, pk.PREC_FP32])
+def test_column_graph_replay_equals_plain_launches(prec):
+    """Per-kernel timing launches plainly; otherwise iterations from the third on replay graphs."""
+    img = images.sphere_pack(22, 0.5, 1.5, 3.5, seed=12)
+    out = []
+    for plain in (True, False):
+        with pk.Solver(base_params(22, Nc_fundamental=4, Kn=0.5, wallExtOrder=1), device=0) as s:
+            s.set_precision(prec)
+            s.setup_physical_grid(img)
+            s.enable_timing(plain)
+            s.iterate(9)
+            out.append((s.get_f()[0], s.chk_converge()))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]

@@ -99,6 +99,26 @@ def test_columns_replay_the_per_node_tasks(n, kw):
     s.close()
 
 
+def test_columns_replay_a_nearly_full_ring():
+    """Plates across an octant's direction: a hyperplane of a column is fluid as a whole behind a
+    solid one, a window of three batches takes 680 of the ring's 685 rows, and the lists are longer
+    than the rows every context reserves for them (which costs the ring its 686th)."""
+    n = 24
+    img = (((np.indices((n, n, n)).sum(0) + 3) % 10) < 5).astype(np.uint8)
+    s = pk.Solver(base_params(n, Nc_fundamental=4, wallExtOrder=1), device=-1)
+    s.setup_physical_grid(img)
+    assert s.geometry_array("wave_info").tolist() == [10, 10, 685, 1200, 680, 816]
+    half = 8 * s.info()["nNodes"]
+    start = np.random.default_rng(3).standard_normal(half + 8 * s.info()["nCorner"])
+    want = start.copy()
+    for t in s.geometry_array("tasks").reshape(-1, 8).tolist():
+        reads = [0.0 if c < 0 else want[(c & ~FW) + (half if c & FW else 0)] for c in t[2:]]
+        row = t[0] * 8 + (t[1] & 7)
+        want[row] = _update(want[row], reads, t[1] >> 3)
+    assert np.array_equal(_replay(s, start.copy()), want)
+    s.close()
+
+
 def test_warps_that_may_leave_meet_on_mbarriers_only():
     """Warps of the column kernel leave one by one once a bounded wait has given up. A counted
     barrier after that point would wait for the ones that left, without a limit: the kernel's only
