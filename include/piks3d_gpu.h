@@ -286,10 +286,10 @@ piks_status piks_run_refined(piks_ctx *ctx, const char *results_path, const char
                              double switch_eps, int32_t *steps32, int32_t *steps, double *permeability,
                              double *seconds);
 
-/* Batches: several solves (contexts with the tile schedule, on one device, of any size,
- * velocity set, Knudsen number and precision) iterated together. One batch iteration runs,
- * per (precision, velocity-chunk) class, a single dataflow launch over the tile jobs of all
- * members, then every member's boundary kernels; after two plain iterations the sequence is
+/* Batches: several solves (contexts with the column or the tile schedule, on one device, of any
+ * size, velocity set, Knudsen number and precision) iterated together. One batch iteration runs,
+ * per (precision, velocity-chunk, schedule) class, a single launch over the columns (or the tile
+ * jobs) of all members, then every member's boundary kernels; after two plain iterations the sequence is
  * captured as a CUDA graph per iteration parity and replayed until the membership changes.
  * Each member's values are those of the same solve run alone. While a context is in a
  * batch, iterate and check it only through the batch. Members may be added and removed

@@ -276,7 +276,7 @@ class Solver:
         _check(self.lib.piks_set_tiles(self._ctx, int(tx), int(ty), int(tz)))
 
     def set_schedule(self, schedule):
-        """SCHED_TILE_DATAFLOW (one launch per sweep) or SCHED_TILE_DIAGONALS."""
+        """SCHED_WAVE (hyperplane columns, the default) or one of the tile forms SCHED_TILE_*."""
         _check(self.lib.piks_set_schedule(self._ctx, int(schedule)))
 
     def autotune(self, candidates=None, sweeps=2):

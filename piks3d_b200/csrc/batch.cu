@@ -1,7 +1,7 @@
 // Batches of solves (piks_batch_*, include/piks3d_gpu.h): several contexts on one device
-// iterated together. One iteration of a batch is, per precision class of its members, one
-// dataflow launch that sweeps every member's tile jobs, followed by each member's boundary
-// kernels. The members' boundary chains are independent of one another, so they fork onto
+// iterated together. One iteration of a batch is, per class of its members (precision, chunk
+// width, columns or tiles), one launch that sweeps every member's columns or tile jobs, followed
+// by each member's boundary kernels. The members' boundary chains are independent of one another, so they fork onto
 // side streams after the sweep and join before the next iteration: in the captured graph they
 // are parallel branches, and small members' launches overlap instead of running one after
 // another. The sequence is captured once as a CUDA graph per iteration parity and replayed

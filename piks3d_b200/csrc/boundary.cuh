@@ -1,8 +1,9 @@
 // Plane kernels of an iteration (x ghosts, inlet / outlet, symmetry), FP64 or FP32 storage.
 //
 // What bounds them: memory round trips; each moves tens of MB. A thread takes one 16-byte piece of
-// all four octants' rows, so that eight loads are in flight per thread and the row lookup is
-// done once. Per iteration on a 128^3 pack of 512 velocities, a thread per
+// all four octants' rows at both ends of the box, so that eight loads are in flight per thread and the
+// row lookup is done once (k_symmetry: of a node's eight rows, four loads for each plane that the
+// node lies on). Per iteration on a 128^3 pack of 512 velocities, a thread per
 // value / this: capture FP64 0.037 / 0.024, FP32 0.033 / 0.015; inlet and outlet 0.037 / 0.024, 0.033 /
 // 0.015; symmetry 0.054 / 0.040, 0.046 / 0.025 ms (some 5 us of each are the launch).
 #pragma once
@@ -83,7 +84,8 @@ __global__ void __launch_bounds__(256) k_inlet_outlet(T *h, const T *ghostW, con
 }
 
 // Specular symmetry planes y = 1, y = Ny, z = 1, z = Nz in the reference's order
-// (solver.F90:1867-1918), on a node's eight values held in registers.
+// (solver.F90:1867-1918): four rows of the node are read and four written per plane, so that a node
+// on an edge of the box sees the first plane's rows in the second.
 template <typename T>
 __global__ void __launch_bounds__(256) k_symmetry(T *h, const int32_t *node, const uint8_t *flag, size_t n, int Nc8) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

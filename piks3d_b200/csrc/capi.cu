@@ -482,12 +482,17 @@ bool build_tiles_for(const piks_ctx *c, const int *dims, int form, TileJobs &tj,
 // cross-section: a batch (one hyperplane of a column) costs some 1000 cycles whatever its size,
 // which asks for wide columns, and its rows fill the ring of one SM's shared memory, which has to
 // hold three of the largest batches and wants some to spare for the loads of the next. With rows
-// of 256 bytes (FP64 32, FP32 64 velocities) that is about 700 rows: 10 x 10, or 9 x 9 where most
-// of the box is pore space and most batches are full. Sweep per iteration on B200: 128^3 pack of
-// porosity 0.40, FP64, 8 x 8 / 10 x 10 / 12 x 12 3.42 / 2.87 / 2.93 ms, FP32 1.71 / 1.48 / 1.67;
-// 100^3 quarter sphere of porosity 0.75, FP64, 8 x 8 / 9 x 9 / 10 x 10 2.50 / 2.54 / 2.69 ms (the
-// tile diagonals 5.31, 2.66 and 5.58 ms). Octants of 8 velocities have rows of a quarter of that
-// and take 12 x 12 (96^3 pack, FP32, 8 x 8 / 10 x 10 / 12 x 12 / 16 x 16: 0.52 / 0.41 / 0.33 / 0.33 ms).
+// of 256 bytes (FP64 32, FP32 64 velocities) that is about 700 rows: 10 x 10, or 9 x 9 from 0.6 of
+// the box swept on, where most batches are full. Sweep per iteration, 8 x 8 / 9 x 9 / 10 x 10, on
+// 100^3 packs of 512 velocities by porosity: FP64 0.4 1.62 / 1.43 / 1.35 ms, 0.5 1.77 / 1.59 / 1.52,
+// 0.6 1.92 / 1.75 / 1.72, 0.7 2.07 / 1.92 / 1.93, 0.85 2.30 / 2.22 / 2.31; FP32 0.4 0.86 / 0.79 /
+// 0.77, 0.5 0.94 / 0.87 / 0.86, 0.6 1.02 / 0.96 / 0.98, 0.7 1.10 / 1.05 / 1.09, 0.85 1.22 / 1.20 /
+// 1.29. So the line lies between 0.5 (FP32) and 0.7 (FP64). 8 x 8 is the better one only in a
+// nearly empty box (quarter sphere, 0.94 swept: FP64 2.36 / 2.44 / 2.66, FP32 1.25 / 1.31 / 1.45)
+// and in small ones (48^3, 0.75: FP64 0.319 / 0.339 / 0.360). 12 x 12 leaves the ring too short
+// (128^3 pack of porosity 0.40, 10 x 10 / 12 x 12: FP64 2.87 / 2.93 ms, FP32 1.48 / 1.67). Octants of 8
+// velocities have rows of a quarter of that and take 12 x 12 (96^3 pack, FP32, 8 x 8 / 10 x 10 /
+// 12 x 12 / 16 x 16: 0.52 / 0.41 / 0.33 / 0.33 ms).
 bool build_wave(piks_ctx *c) {
   c->wave = WaveJobs{};
   const int Nc8 = c->vel.Nc8;

@@ -343,11 +343,12 @@ __host__ __device__ constexpr int wall_doubles(int LPW, int Nc8, int far_rows) {
 // densities are summed serially over l in the reference's order, a lane per face, and the
 // re-emission reads the extrapolated values on chip (WPlan); a face value is stored only where it
 // is the slot's final content. Same operations on the same operands as k_walls, in the same order.
-// The far point's rows are read where its coefficient is not 0 (wallExtOrder 1 makes it 0).
+// The far point's rows are read where its coefficient is not 0 (wallExtOrder 1 makes it 0; a far value
+// that has overflowed then reaches the wall's node by the next sweep, not as 0 * inf at the wall).
 // What bounds it: the rows' bytes (2.1 GB a pass on a 128^3 pack of 300,000 walls, 512
 // velocities, 0.33 ms at the copy rate) with 29 walls of 7.6 KB on an SM. A warp that took face
-// after face, each a load round trip and a serial sum, needed 0.595 ms; this needs 0.40. With 1728
-// velocities (75 x 53 x 37 pack, 20,000 walls), where the rows went through L2 twice, 0.476 -> 0.119 ms.
+// after face, each a load round trip and a serial sum, needed 0.595 ms; this needs 0.40. With 216
+// velocities an octant (75 x 53 x 37 pack, 20,000 walls), where the rows went through L2 twice, 0.476 -> 0.119 ms.
 template <int LPW>
 __global__ void __launch_bounds__(LPW <= 32 ? 32 : LPW, LPW <= 32 ? 26 : LPW == 128 ? 8 : 3)
 k_walls_rows(const DevState a, int begin, int end, int gbuf, int far_rows) {
@@ -962,7 +963,7 @@ void launch_walls_rows(const DevState &s, int begin, int end, int gbuf, cudaStre
 }
 }  // namespace
 
-// Octants of 8, 64, 216 and 512 velocities keep a wall's rows on chip; 1728 and more do not fit.
+// Octants of 8, 64, 216 and 512 velocities keep a wall's rows on chip; those of 1728 and 4096 do not fit.
 void launch_walls(const DevState &s, int begin, int end, int gbuf, cudaStream_t st) {
   if (end <= begin) return;
   if (g_plan_ok && s.Nc8 <= 512 && s.Nc8 % 8 == 0) {
