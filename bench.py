@@ -297,7 +297,7 @@ def traffic_per_update(precision):
     """DRAM bytes per swept voxel-velocity update of the sweep kernel, from the committed
     summary of an ncu capture (profiles/), or None."""
     try:
-        d = json.load(open(os.path.join(ROOT, "profiles", "tile_sweep_traffic.json")))
+        d = json.load(open(os.path.join(ROOT, "profiles", "sweep_traffic.json")))
         return d[precision]["dram_bytes_per_swept_update"]
     except Exception:
         return None

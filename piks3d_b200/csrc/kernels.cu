@@ -343,8 +343,8 @@ __host__ __device__ constexpr int wall_doubles(int LPW, int Nc8, int far_rows) {
 // densities are summed serially over l in the reference's order, a lane per face, and the
 // re-emission reads the extrapolated values on chip (WPlan); a face value is stored only where it
 // is the slot's final content. Same operations on the same operands as k_walls, in the same order.
-// The far point's rows are read where its coefficient is not 0 (wallExtOrder 1 makes it 0; a far value
-// that has overflowed then reaches the wall's node by the next sweep, not as 0 * inf at the wall).
+// The far point's rows are read where its coefficient is not 0 (wallExtOrder 1 makes it 0; the near
+// point is downwind of it, so the sweep has made the near value not finite where the far one is).
 // What bounds it: the rows' bytes (2.1 GB a pass on a 128^3 pack of 300,000 walls, 512
 // velocities, 0.33 ms at the copy rate) with 29 walls of 7.6 KB on an SM. A warp that took face
 // after face, each a load round trip and a serial sum, needed 0.595 ms; this needs 0.40. With 216
