@@ -32,12 +32,14 @@
 // (FP32) rows per swept row, each CTA as one chain of metadata, rows, ten to fourteen local
 // hyperplanes with a few tasks each, and write-back. Here a hyperplane of a column holds
 // tens of tasks, the loads of the next ones run meanwhile, and about 1.5 rows are staged. What is
-// left is some 1000 cycles a batch for the hand-over to the next hyperplane, and 31 a task (the
-// consumers' shared-memory reads); short columns wait for the chain of upwind columns. Sweep per
-// iteration, tile diagonals / this: 128^3 pack, 512 velocities, FP64 5.31 / 2.79 ms, FP32 2.66 / 1.45;
-// 100^3 quarter sphere FP64 5.58 / 2.49; 48^3 pack FP64 0.598 / 0.271; 256^3 field of porosity 0.20,
-// FP32, 8.98 / 6.69; 96^3 pack, 64 velocities, FP32 0.72 / 0.32; 75 x 53 x 37, 1728 velocities, FP64
-// 2.28 / 0.96.
+// left is some 930 cycles a batch for the hand-over to the next hyperplane, and 30 (FP64) to 32 (FP32)
+// a task, whose shared-memory accesses are 35 and 33 wavefronts (fitted over packs of five porosities
+// with 7 x 7 and 8 x 8 columns; wider ones take 4 to 25 % more, as the ring no longer holds the next
+// batches' rows); short columns wait for the chain of upwind columns. Sweep per iteration, tile
+// diagonals / this: 128^3 pack, 512 velocities, FP64 5.31 / 2.70 ms, FP32 2.66 / 1.43; 100^3 quarter
+// sphere FP64 5.58 / 2.43; 48^3 pack FP64 0.598 / 0.256; 256^3 field of porosity 0.20, FP32, 8.98 /
+// 6.55; 96^3 pack, 64 velocities, FP32 0.72 / 0.316; 75 x 53 x 37, 216 velocities an octant, FP64 2.28 /
+// 0.95.
 #include <cuda_runtime.h>
 
 #include <algorithm>
