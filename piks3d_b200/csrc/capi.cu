@@ -327,7 +327,7 @@ void drain_timing(piks_ctx *c) {
   c->ev_next = 0;
 }
 
-// The tile sweeps' error flag: set when a dependency wait or a staging wait gave up (the
+// The sweep's error flag: set when a dependency wait or a staging wait gave up (the
 // values of that sweep are then not the solver's).
 piks_status check_sweep_error(piks_ctx *c) {
   const int *flag = c->use_wave ? c->ds.wv.err : c->use_tiles ? c->ds.tv.err : nullptr;
@@ -598,8 +598,8 @@ piks_status upload_tiles(piks_ctx *c) {
     if (p) release(c, const_cast<void *>(p));
   tv = TileView{};
   piks_status st;
-  if (c->use_wave && c->tiles.row_count.empty()) return PIKS_OK;
-  if (!c->use_tiles && !c->use_wave) {
+  if (c->use_wave) return PIKS_OK;
+  if (!c->use_tiles) {
     // the per-node hyperplane sweep reads the task list (uploaded once, only if needed)
     if (!c->ds.tasks) {
       int32_t *pt = nullptr;
