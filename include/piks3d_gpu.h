@@ -286,7 +286,7 @@ piks_status piks_run_refined(piks_ctx *ctx, const char *results_path, const char
                              double switch_eps, int32_t *steps32, int32_t *steps, double *permeability,
                              double *seconds);
 
-/* Batches: several solves (contexts with the column or the tile schedule, on one device, of any
+/* Batches: several solves (contexts on columns, tile diagonals or dataflow, on one device, of any
  * size, velocity set, Knudsen number and precision) iterated together. One batch iteration runs,
  * per (precision, velocity-chunk, schedule) class, a single launch over the columns (or the tile
  * jobs) of all members, then every member's boundary kernels; after two plain iterations the sequence is

@@ -89,12 +89,16 @@ void drop_graphs(piks_batch *b) {
 // Device copies of the members' states and, per (precision, V) class, the work items of the
 // merged sweep: ordered by tile diagonal, then member, then the member's launch order, then
 // velocity chunk, so that every item's upstream items come before it.
+// Whether a batch launch can sweep the context: on columns, or on tile jobs in the slot form (the
+// split forms have no launch plan to take the items from).
+bool sweepable(const piks_ctx *c) { return c->use_wave || (c->use_tiles && !c->tiles.split); }
+
 piks_status rebuild(piks_batch *b) {
   drop_graphs(b);
   b->warm = 0;
   const size_t nm = b->members.size();
   for (const piks_ctx *c : b->members)
-    if (!c->use_wave && !c->use_tiles) return fail(PIKS_ERR_STATE, "a batch member no longer has a column or tile schedule");
+    if (!sweepable(c)) return fail(PIKS_ERR_STATE, "a batch member no longer has a schedule that a batch sweeps");
   if (nm > b->states_cap) {
     if (b->d_states) cudaFree(b->d_states);
     b->d_states = nullptr;
@@ -279,7 +283,7 @@ piks_status piks_batch_add(piks_batch *b, piks_ctx *c) {
   if (!b || !c) return fail(PIKS_ERR_ARG, "null argument");
   if (!c->have_geometry) return fail(PIKS_ERR_STATE, "batch member has no device state");
   if (c->device != b->device) return fail(PIKS_ERR_ARG, "batch member lives on another device");
-  if (!c->use_tiles && !c->use_wave) return fail(PIKS_ERR_ARG, "batch members need the column or the tile schedule");
+  if (!sweepable(c)) return fail(PIKS_ERR_ARG, "batch members need the column schedule or tile diagonals / dataflow");
   if (c->setup.nranks > 1) return fail(PIKS_ERR_ARG, "a slab of a decomposed box cannot join a batch");
   if (b->members.size() >= 4096) return fail(PIKS_ERR_ARG, "batch holds at most 4096 members");
   if (std::find(b->members.begin(), b->members.end(), c) != b->members.end()) return PIKS_OK;

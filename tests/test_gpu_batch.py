@@ -121,3 +121,31 @@ def test_batch_with_216_velocity_members_equals_alone():
         for s in ss:
             b.remove(s)
             s.close()
+
+
+def test_batch_takes_the_schedules_it_can_sweep():
+    """Columns and tile diagonals / dataflow are swept in a batch (values as alone). Per-node and
+    split-form contexts have no items for its launch: they are refused, also when a member moves to
+    such a schedule."""
+    make, kw, prec = MEMBERS[1]
+    img = make()
+    alone, _ = list(_alone(1, {4}).values())[0]
+    for sched in (pk.SCHED_WAVE, pk.SCHED_TILE_DIAGONALS, pk.SCHED_TILE_DATAFLOW, pk.SCHED_TILE_COLUMNS,
+                  pk.SCHED_TILE_PIPELINED, None):
+        with pk.Batch(device=0) as b, pk.Solver(base_params(img.shape[0], **kw), device=0) as s:
+            s.set_tiles(*((4, 4, 4) if sched is not None else (0, 0, 0)))
+            if sched is not None:
+                s.set_schedule(sched)
+            s.setup_physical_grid(img)
+            if sched in (pk.SCHED_TILE_COLUMNS, pk.SCHED_TILE_PIPELINED, None):
+                with pytest.raises(pk.PiksError):
+                    b.add(s)
+                continue
+            b.add(s)
+            b.iterate(4)
+            b.synchronize()
+            assert np.array_equal(s.get_f()[0], alone)
+            s.set_schedule(pk.SCHED_TILE_COLUMNS)
+            with pytest.raises(pk.PiksError):
+                b.iterate(1)
+            b.remove(s)
