@@ -13,7 +13,6 @@
 #include <mutex>
 #include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -211,17 +210,8 @@ cudaError_t fetch_macro(piks_ctx *c, double *const dst[4]) {
     }
     cudaEventDestroy(done);
   };
-  std::vector<std::thread> th;
-  if (marked == cudaSuccess) {
-    th.reserve((size_t)nw);
-    for (int w = 1; w < nw; ++w) {
-      try { th.emplace_back(work, w); } catch (const std::system_error &) { break; }  // the others take its blocks
-    }
-    work(0);
-    for (auto &t : th) t.join();
-  } else {
-    status = (int)marked;
-  }
+  if (marked == cudaSuccess) on_threads(nw, work);
+  else status = (int)marked;
   if (computed) cudaEventDestroy(computed);
   g_macro_stages.give(pinned);
   return (cudaError_t)status.load();
@@ -941,9 +931,12 @@ piks_status piks_setup_physical_grid(piks_ctx *c, const uint8_t *raw, int64_t nb
     const int slots = tile_slots(c, c->tiles_next_dims);
     (void)slots;
     const int form = tile_form(c->schedule);
-    c->tiles_next_ready = std::async(std::launch::async, [c, form] {
-      return build_tiles_for(c, c->tiles_next_dims, form, c->tiles_next, PIKS_PREC_FP64);
-    });
+    try {
+      c->tiles_next_ready = std::async(std::launch::async, [c, form] {
+        return build_tiles_for(c, c->tiles_next_dims, form, c->tiles_next, PIKS_PREC_FP64);
+      });
+    } catch (const std::exception &) {  // no thread to be had: built at the switch
+    }
   }
   c->mass = 1.0;  // flow.F90:97
   c->error = 1.0;

@@ -711,9 +711,7 @@ piks_status finish_geometry(const Setup &s, Geometry &g, std::string &err) {
           }
         }
       }
-      std::vector<std::thread> th;
-      for (int o = 0; o < 8; ++o) th.emplace_back(sweep_octant, o, pass, &fill[(size_t)o]);
-      for (auto &t : th) t.join();
+      on_threads(8, [&](int o) { sweep_octant(o, pass, &fill[(size_t)o]); });
     }
   }
 

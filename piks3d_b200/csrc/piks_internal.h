@@ -1,16 +1,33 @@
 // Internal host-side structures of libpiks3d_b200 (not part of the C ABI).
 #pragma once
 #include <cstdint>
+#include <exception>
 #include <functional>
 #include <memory>
 #include <new>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
 #include "piks3d_gpu.h"
 
 namespace piks {
+
+// Runs fn(0) .. fn(n - 1) on n threads, the last on the calling one; where the system gives no
+// more threads, the calling one runs what is left.
+template <typename F>
+void on_threads(int n, F fn) {
+  std::vector<std::thread> th;
+  int i = 0;
+  try {
+    th.reserve((size_t)(n > 1 ? n - 1 : 0));
+    for (; i < n - 1; ++i) th.emplace_back([&fn, i] { fn(i); });
+  } catch (const std::exception &) {
+  }
+  for (; i < n; ++i) fn(i);
+  for (auto &t : th) t.join();
+}
 
 // std::allocator that leaves new elements uninitialised: for the large host arrays that
 // are written in full right after they are sized (their pages are then first touched by

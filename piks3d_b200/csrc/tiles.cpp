@@ -23,13 +23,7 @@ template <typename F>
 void parallel_chunks_indexed(int64_t n, F fn) {
   const int nt = chunk_count(n);
   if (nt <= 1) { fn(0, (int64_t)0, n); return; }
-  std::vector<std::thread> th;
-  th.reserve((size_t)nt);
-  for (int i = 0; i < nt; ++i) {
-    const int64_t b = n * i / nt, e = n * (i + 1) / nt;
-    th.emplace_back([=, &fn] { fn(i, b, e); });
-  }
-  for (auto &t : th) t.join();
+  on_threads(nt, [&fn, n, nt](int i) { fn(i, n * i / nt, n * (i + 1) / nt); });
 }
 
 // Runs fn(begin, end) over [0, n) split into contiguous chunks on up to 16 threads.
@@ -353,9 +347,7 @@ bool build_tile_jobs(const Geometry &g, int TX, int TY, int TZ, int max_slots, T
       }
     };
     if (ntask < 4096) { for (int o = 0; o < 8; ++o) run(o); return; }
-    std::vector<std::thread> th;
-    for (int o = 0; o < 8; ++o) th.emplace_back([&run, o] { run(o); });
-    for (auto &x : th) x.join();
+    on_threads(8, run);
   };
   // jobs = non-empty pairs, ordered by (diagonal * 8 + octant), then tile (counting sort)
   const int64_t npairs = ntiles * 8;

@@ -14,15 +14,6 @@ int worker_count() {
   return (int)std::max(1u, std::min(hw ? hw : 1u, 16u));
 }
 
-// Runs fn(worker) on `n` threads.
-template <typename F>
-void on_workers(int n, F fn) {
-  if (n <= 1) { fn(0); return; }
-  std::vector<std::thread> th;
-  for (int i = 0; i < n; ++i) th.emplace_back([&fn, i] { fn(i); });
-  for (auto &t : th) t.join();
-}
-
 constexpr int kFw = 1 << 30;
 
 // A row that a column holds: its code and where it stands (batch, list, index in the list).
@@ -208,7 +199,7 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   const int nw = ntask < 4096 ? 1 : worker_count();
   const int64_t nnode = (int64_t)g.node_g.size(), GX = g.GX, GXY = (int64_t)g.GX * g.GY;
   wb.xyz.resize((size_t)nnode);
-  on_workers(nw, [&](int t) {
+  on_threads(nw, [&](int t) {
     for (int64_t n = nnode * t / nw; n < nnode * (t + 1) / nw; ++n) {
       const int64_t gi = g.node_g[(size_t)n];
       wb.xyz[(size_t)n] = (uint64_t)(gi % GX) | (uint64_t)(gi / GX % g.GY) << 21 | (uint64_t)(gi / GXY) << 42;
@@ -226,7 +217,7 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   };
   BigVec<int32_t> key((size_t)ntask);
   std::vector<std::vector<int32_t>> count((size_t)nw, std::vector<int32_t>((size_t)nkeys, 0));
-  on_workers(nw, [&](int t) {
+  on_threads(nw, [&](int t) {
     auto &c = count[(size_t)t];
     for (int64_t q = ntask * t / nw; q < ntask * (t + 1) / nw; ++q) c[(size_t)(key[(size_t)q] = key_of(q))]++;
   });
@@ -246,7 +237,7 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   }
   const int ncol = wj.ncol = (int)wb.key_of_col.size();
   wb.order.resize((size_t)ntask);
-  on_workers(nw, [&](int t) {
+  on_threads(nw, [&](int t) {
     auto &c = count[(size_t)t];
     for (int64_t q = ntask * t / nw; q < ntask * (t + 1) / nw; ++q) wb.order[(size_t)c[(size_t)key[(size_t)q]]++] = (int32_t)q;
   });
@@ -280,7 +271,7 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   wb.scratch.resize((size_t)nw);
   wb.rows_at.resize((size_t)ncol);
   std::atomic<int> next{0};
-  on_workers(nw, [&](int t) {
+  on_threads(nw, [&](int t) {
     wb.scratch[(size_t)t].cell.assign((size_t)4 * (A + 2) * (B + 2) * 3, Held{-1, 0, 0});
     for (int col; (col = next.fetch_add(1)) < ncol;) wb.scan(col, t);
   });
@@ -316,7 +307,7 @@ bool build_wave_jobs(const Geometry &g, int A, int B, const std::function<int(in
   if (wj.ring < win_rows) return false;
   wj.rows.resize((size_t)groups * 4);
   next = 0;
-  on_workers(nw, [&](int) {
+  on_threads(nw, [&](int) {
     for (int col; (col = next.fetch_add(1)) < ncol;) wb.place(col);
   });
   // columns in dependency order: by the x + y column diagonal of the octant's frame

@@ -5,6 +5,8 @@ another in their listed order - and every swept row must equal the per-node task
 bit for bit."""
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -151,3 +153,47 @@ def test_schedule_reports_what_is_in_use():
     s.setup_physical_grid(np.ones((12, 12, 12), np.uint8))   # nothing to sweep: no columns are built
     assert s.schedule()["launch"] != pk.SCHED_WAVE and s.schedule()["columns"] == 0
     s.close()
+
+
+_NO_THREADS = """
+import hashlib, os, resource, sys
+sys.path[:0] = [%r, %r]
+import numpy as np
+import piks3d_b200 as pk
+from conftest import base_params
+from piks3d_b200 import images
+img = images.sphere_pack(30, 0.5, 1.5, 3.5, seed=4)
+def digests():
+    out = []
+    for tiles in (None, (4, 4, 4)):
+        s = pk.Solver(base_params(30, Nc_fundamental=4), device=-1)
+        if tiles:
+            s.set_tiles(*tiles)
+        s.setup_physical_grid(img)
+        for name in ("tasks", "tile_rows", "tile_tasks") + (() if tiles else ("wave_rows", "wave_tasks", "wave_batch", "wave_cols")):
+            out.append(hashlib.sha256(s.geometry_array(name).tobytes()).hexdigest())
+        s.close()
+    return out
+want = digests()
+if os.getuid() == 0:
+    os.setuid(65534)                   # the limit does not hold for root
+resource.setrlimit(resource.RLIMIT_NPROC, (0, 0))
+import threading
+try:
+    threading.Thread(target=int).start()
+    print("unlimited")
+except RuntimeError:
+    print("limited")
+print("same" if digests() == want else "different")
+"""
+
+
+def test_setup_without_threads_to_be_had():
+    """A process that may start no thread sets images up on the one it has, with the same result."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", _NO_THREADS % (os.path.dirname(here), here)], capture_output=True, text=True,
+                       timeout=300)
+    out = r.stdout.split()
+    if out[:1] == ["unlimited"]:
+        pytest.skip("the thread limit does not hold here")
+    assert r.returncode == 0 and out == ["limited", "same"], (r.returncode, r.stdout, r.stderr[-800:])
